@@ -1,6 +1,6 @@
-"""Grid search with the misfit bound (many events, L2): the optimum, origin
-time and misfit are the full search's bit for bit, whatever the bound rules
-out -- graded and skipped picks, tables with infinities, ties, grids around
+"""Grid search with the misfit bounds.  L2 (many events): the optimum, origin
+time and misfit are the full search's bit for bit; L1: the FP64 exhaustive
+search's up to the FP32 ranking, whatever the bound rules out -- graded and skipped picks, tables with infinities, ties, grids around
 the size and event count from which the bound is used, every table width."""
 import numpy as np
 import pytest
@@ -48,4 +48,37 @@ def test_bounded_search_matches_oracle_bitwise(fk, ntf, nz, nx, ny, nev, kind):
     for e in range(nev):
         want = _oracle(tables, picks[e], wts[e])
         assert (oi[e], t0[e], ob[e]) == want, e
+    loc.finalize()
+
+
+@pytest.mark.parametrize("ntf,nz,nx,ny,nev", [(1, 16, 17, 16, 3), (2, 16, 16, 16, 17), (16, 17, 16, 16, 8),
+                                              (17, 21, 19, 23, 33), (45, 16, 16, 15, 7), (64, 25, 31, 29, 20)])
+@pytest.mark.parametrize("kind", ["times", "random"])
+def test_bounded_l1_matches_fp64_exhaustive(fk, ntf, nz, nx, ny, nev, kind):
+    ngrd = nz * nx * ny
+    rng = np.random.default_rng(ntf * 10 + nev)
+    if kind == "times":
+        tables = station_tables(nz, nx, ny, 100.0, ntf, seed=ntf)
+    else:
+        tables = rng.uniform(0.5, 12.0, (ntf, ngrd)).astype(np.float32)
+    _, picks = synthetic_events(tables, nev, seed=ntf + 2)
+    wts = np.full(picks.shape, 0.5)
+    wts[rng.random(picks.shape) < 0.15] = 0.0
+    wts[:, 0] = 0.5
+    loc = fk.Locator(nev, ntf, ngrd)
+    for k in range(ntf):
+        loc.setTravelTimeField32f(k + 1, tables[k])
+    for e in range(nev):
+        loc.setObservation(e + 1, np.arange(1, ntf + 1), picks[e], wts[e])
+    loc.setNorm(1)
+    oi, t0, ob = loc.locateEvents(np.arange(1, nev + 1))
+    for e in range(nev):
+        red = picks[e] - picks[e].max()
+        _, _, gob = O.locate_l1_best64(tables, red, wts[e])
+        _, t_here, ob_here = O.locate_l1_best64(tables[:, [oi[e] - 1]], red, wts[e])
+        # the FP32 ranking misfit is off by at most (N + 1) 2^-24 sum (|o| + |T|), both points
+        off = 2 * 65 * 2.0 ** -24 * 0.5 * (np.abs(red).sum() + np.abs(tables).max(1).sum())
+        assert ob_here <= gob + off, (e, ob_here, gob)
+        assert abs(ob[e] - ob_here) <= 1e-9 * max(ob_here, 1e-12)
+        assert abs(t0[e] - (t_here + picks[e].max())) <= 1e-9 * max(1.0, abs(t0[e]))
     loc.finalize()
