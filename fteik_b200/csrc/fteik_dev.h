@@ -123,6 +123,14 @@ int fk2d_solve(int fsm, const fk_grid2d_t *grids, const fk_work2d_t *work,
                fk_result3d_t *results, int nwork, int max_nx, int max_nz, double eps,
                int nsweep, double conv_tol, int max_pass, cudaStream_t stream);
 
+/* The same, LSM or FSM, on one grid (host struct) by the diagonal walk, where
+ * fk2d_diag_bytes says that it applies: nsweep passes, device scratch of
+ * *model + nwork * *source bytes, the model's part kept between calls unless
+ * set_model. */
+int fk2d_diag_bytes(int nz, int nx, size_t *model, size_t *source);
+int fk2d_solve_diag(const fk_grid2d_t *grid, const fk_work2d_t *work, fk_result3d_t *results, int nwork,
+                    double eps, int nsweep, void *scratch, int set_model, cudaStream_t stream);
+
 /* 2D ray paths (rays2d.cu): pass 1 counts points and (cell, length) pieces
  * and writes npts / nseg / status / tn / tne per ray; pass 2 writes the
  * points and pieces at pts_off / seg_off.  Positions relative to the model

@@ -29,6 +29,8 @@ static struct {
     double *rec_all;      /* device [cap][nrec] */
     int rec_cap;
     double *gx, *gz;      /* device [ngrd] gradient of the current field */
+    void *diag;           /* diagonal walk's scratch (fk2d_solve_diag) */
+    size_t diag_cap;
     bool have_grad;
 } S2;
 
@@ -55,6 +57,7 @@ void fteik_solver2d_free(void)
     fk_dfree(S2.grid_dev); fk_dfree(S2.work_dev); fk_dfree(S2.res_dev);
     fk_dfree(S2.tt_all); fk_dfree(S2.work_all); fk_dfree(S2.res_all); fk_dfree(S2.fptr_dev);
     fk_dfree(S2.rec_all); fk_dfree(S2.gx); fk_dfree(S2.gz);
+    fk_dfree(S2.diag);
     free(S2.tt_rec);
     memset(&S2, 0, sizeof(S2));
     S2.src = -1;
@@ -176,6 +179,33 @@ static void set_work(fk_work2d_t *w, int isrc, double *tt)
     w->tt = tt;
 }
 
+/* Solve n work items of one grid (g, also at grid_dev): by the diagonal walk
+ * where it applies, in pieces of at most 1 GiB of field copies. */
+static int run_solve(int fsm, const fk_grid2d_t *g, const fk_work2d_t *work, fk_result3d_t *res, int n, cudaStream_t s,
+                     const char *who)
+{
+    size_t model, source;
+    if (!fk2d_diag_bytes(g->nz, g->nx, &model, &source))
+        /* solver2D.F90:935-946: the reference's test never stops early */
+        return fk2d_solve(fsm, S2.grid_dev, work, res, n, g->nx, g->nz, S2.eps, S2.nsweep, -1.0, 0, s);
+    size_t most = ((size_t)1 << 30) / source;
+    if (most < 1) most = 1;
+    if (most > (size_t)n) most = (size_t)n;
+    const size_t need = model + most * source;
+    if (need > S2.diag_cap) {
+        fk_dfree(S2.diag);
+        S2.diag = fk_dalloc(need, who);
+        S2.diag_cap = S2.diag ? need : 0;
+        if (!S2.diag) return (int)cudaErrorMemoryAllocation;
+    }
+    int e = 0;
+    for (int i = 0; !e && i < n; i += (int)most) {
+        const int m = n - i < (int)most ? n - i : (int)most;
+        e = fk2d_solve_diag(g, work + i, res + i, m, S2.eps, S2.nsweep, S2.diag, i == 0, s);
+    }
+    return e;
+}
+
 static int solve_one(int isrc, int fsm, const char *who)
 {
     S2.have_times = false;
@@ -201,9 +231,7 @@ static int solve_one(int isrc, int fsm, const char *who)
     fk_result3d_t res;
     int e = (int)cudaMemcpyAsync(S2.grid_dev, &g, sizeof(g), cudaMemcpyHostToDevice, s);
     if (!e) e = (int)cudaMemcpyAsync(S2.work_dev, &w, sizeof(w), cudaMemcpyHostToDevice, s);
-    /* solver2D.F90:935-946: the reference's test never stops early */
-    if (!e) e = fk2d_solve(fsm, S2.grid_dev, S2.work_dev, S2.res_dev, 1, nx, nz, S2.eps, S2.nsweep,
-                          -1.0, 0, s);
+    if (!e) e = run_solve(fsm, &g, S2.work_dev, S2.res_dev, 1, s, who);
     if (!e) e = (int)cudaMemcpyAsync(&res, S2.res_dev, sizeof(res), cudaMemcpyDeviceToHost, s);
     if (!e) e = (int)cudaStreamSynchronize(s);
     if (fk_check(e, who) || res.status) return 1;
@@ -301,8 +329,7 @@ static int solve_chunks(const char *who)
         }
         e = (int)cudaMemcpyAsync(S2.work_all, w, sizeof(fk_work2d_t) * (size_t)n, cudaMemcpyHostToDevice, s);
         if (!e) e = (int)cudaMemcpyAsync(S2.fptr_dev, fp, sizeof(void *) * (size_t)n, cudaMemcpyHostToDevice, s);
-        /* solver2D.F90:935-946: the reference's test never stops early */
-        if (!e) e = fk2d_solve(0, S2.grid_dev, S2.work_all, S2.res_all, n, nx, nz, S2.eps, S2.nsweep, -1.0, 0, s);
+        if (!e) e = run_solve(0, &g, S2.work_all, S2.res_all, n, s, who);
         if (!e && nrec > 0)
             e = fk_receivers_batch2d(nx, zp, fk_model.dz, fk_model.dx, S2.fptr_dev, n, nrec, fk_receiver.ri_dev,
                                      fk_receiver.rd_dev, S2.rec_all, s);
