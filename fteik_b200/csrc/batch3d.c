@@ -55,7 +55,7 @@ static struct {
     fk_slabplan_t plan;     /* slab-pipelined schedule */
     int spin_epoch;         /* poll limit the plan (and graph) was built with */
     int cfg_epoch;          /* slab configuration the plan (and graph) was built with */
-    int tuned[6];           /* configuration in use: staged, pairs, progress, blocks/SM passes, init, init pairs */
+    int tuned[7];           /* configuration in use: staged, pairs, progress, blocks/SM passes, init, init pairs, tiles */
     float tune_ms[2];       /* its init / pass kernel times when tuned (0: not timed) */
     int tune_runs;          /* candidate solves the last tuning ran (0: cache hit or nothing to tune) */
     bool work_dirty;        /* source positions changed, shape unchanged */
@@ -435,14 +435,19 @@ static int build_work(const char *who)
  * eagerly, with CUDA events around each kernel:
  *   1. staged x pairs x progress (8 | 32), all resident blocks;
  *   2. the best of 1 at 3 and 2 resident blocks per SM;
+ *   3. with every knob left to the library, the tile schedule (tile3d.cu) if
+ *      it holds the work list in at most TILE_LAUNCHES launches;
  * the pass kernel takes the fastest pass time, the initialisation kernel the
- * blocks per SM of the fastest initialisation time.  Every candidate is run
+ * blocks per SM of the fastest initialisation time; the tile schedule, one
+ * kernel for both, takes their place if it beats the two together.  Every candidate is run
  * twice and timed by its faster run.  Every configuration gives the same
  * fields bit for bit, so the search changes only the time.  The choice is
  * kept per work list (grid shapes, sources per grid, precision, passes) in
  * memory and, when FTEIK_B200_TUNE_CACHE names a file, in that file, so
  * later processes skip the search. */
-static void tune_apply(const int t[6])
+#define TILE_LAUNCHES 8
+
+static void tune_apply(const int t[7])
 {
     SB.plan.dev.staged = SB.precision == 4 && t[0] == 1;
     SB.plan.dev.pairs = t[1] ? SB.plan.pairs_all : NULL;
@@ -450,6 +455,7 @@ static void tune_apply(const int t[6])
     SB.plan.dev.blocks_per_sm = t[3];
     SB.plan.dev.init_blocks_per_sm = t[4];
     SB.plan.dev.init_pairs = (SB.precision == 4 && t[5]) ? SB.plan.pairs_all : NULL;
+    SB.plan.dev.use_tiles = t[6] && SB.plan.have_tiles;
     memcpy(SB.tuned, t, sizeof(SB.tuned));
 }
 
@@ -472,37 +478,41 @@ static void tune_key(char *key, size_t cap)
 
 #define TUNE_MEM 16
 static char g_tune_key[TUNE_MEM][512];
-static int g_tune_val[TUNE_MEM][6];
+static int g_tune_val[TUNE_MEM][7];
 static int g_tune_n = 0;
 
-static int tune_lookup(const char *key, int t[6])
+static int tune_lookup(const char *key, int t[7])
 {
     for (int i = 0; i < g_tune_n; i++)
-        if (strcmp(g_tune_key[i], key) == 0) { memcpy(t, g_tune_val[i], 6 * sizeof(int)); return 1; }
+        if (strcmp(g_tune_key[i], key) == 0) { memcpy(t, g_tune_val[i], 7 * sizeof(int)); return 1; }
     const char *path = getenv("FTEIK_B200_TUNE_CACHE");
     if (!path || !*path) return 0;
     FILE *f = fopen(path, "r");
     if (!f) return 0;
     char line[700], k[600];
     int found = 0;
-    while (fgets(line, sizeof(line), f))
-        if (sscanf(line, "%599s %d %d %d %d %d %d", k, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5]) == 7 &&
-            strcmp(k, key) == 0)
-            found = 1;   /* the last line for a key wins */
+    while (fgets(line, sizeof(line), f)) {
+        int v[7] = {0};   /* lines written before the tile schedule have six values */
+        if (sscanf(line, "%599s %d %d %d %d %d %d %d", k, &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6]) >= 7 &&
+            strcmp(k, key) == 0) {
+            memcpy(t, v, sizeof(v));
+            found = 1;    /* the last line for a key wins */
+        }
+    }
     fclose(f);
     return found;
 }
 
-static void tune_store(const char *key, const int t[6])
+static void tune_store(const char *key, const int t[7])
 {
     const int i = g_tune_n < TUNE_MEM ? g_tune_n++ : TUNE_MEM - 1;
     snprintf(g_tune_key[i], sizeof(g_tune_key[i]), "%s", key);
-    memcpy(g_tune_val[i], t, 6 * sizeof(int));
+    memcpy(g_tune_val[i], t, 7 * sizeof(int));
     const char *path = getenv("FTEIK_B200_TUNE_CACHE");
     if (!path || !*path) return;
     FILE *f = fopen(path, "a");
     if (!f) return;
-    fprintf(f, "%s %d %d %d %d %d %d\n", key, t[0], t[1], t[2], t[3], t[4], t[5]);
+    fprintf(f, "%s %d %d %d %d %d %d %d\n", key, t[0], t[1], t[2], t[3], t[4], t[5], t[6]);
     fclose(f);
 }
 
@@ -538,9 +548,9 @@ static int tune(const char *who)
 {
     const fk_slabcfg_t cfg = fk_slabcfg();
     /* a knob at 0 is explicit: progress by task count, all resident blocks */
-    int t[6] = {SB.precision == 4 && cfg.staged == 1, cfg.pairs != 0, cfg.progress > 0 ? cfg.progress : 0,
+    int t[7] = {SB.precision == 4 && cfg.staged == 1, cfg.pairs != 0, cfg.progress > 0 ? cfg.progress : 0,
                 cfg.blocks_per_sm > 0 ? cfg.blocks_per_sm : 0, cfg.blocks_per_sm > 0 ? cfg.blocks_per_sm : 0,
-                SB.precision == 4 && cfg.pairs != 0};
+                SB.precision == 4 && cfg.pairs != 0, 0};
     SB.tune_ms[0] = SB.tune_ms[1] = 0.0f;
     SB.tune_runs = 0;
     const bool search = (cfg.staged < 0 && SB.precision == 4) || cfg.pairs < 0 || cfg.progress < 0 ||
@@ -548,7 +558,15 @@ static int tune(const char *who)
     if (!search) { tune_apply(t); return 0; }
     char key[512];
     tune_key(key, sizeof(key));
-    if (tune_lookup(key, t)) { tune_apply(t); return 0; }
+    const bool tiles = cfg.staged < 0 && cfg.pairs < 0 && cfg.progress < 0 && cfg.blocks_per_sm < 0;
+    const int conv = SB.conv_tol >= 0.0 && SB.max_pass > 0;
+    if (tune_lookup(key, t)) {
+        /* the knobs left open are part of the choice: a set one rules out the tiles */
+        if (!tiles) t[6] = 0;
+        if (t[6] && fk_slabplan_tiles(&SB.plan, SB.precision, conv, who)) return 1;
+        tune_apply(t);
+        return 0;
+    }
     if (ensure_events()) { FK_ERR("%s: cannot create events", who); return 1; }
     const int st_n = (cfg.staged < 0 && SB.precision == 4) ? 2 : 1;
     const int pr_n = cfg.pairs < 0 ? 2 : 1;
@@ -556,12 +574,12 @@ static int tune(const char *who)
     /* the two kernels are chosen apart: the passes by their time, the
      * initialisation sweeps (pairs, blocks per SM) by theirs */
     float best_pass = 3.4e38f, best_init = 3.4e38f;
-    int best[6], best_i[2] = {t[4], t[5]};
+    int best[7], best_i[2] = {t[4], t[5]};
     memcpy(best, t, sizeof(best));
     for (int a = 0; a < st_n * pr_n * ch_n; a++) {
         const int pr = pr_n == 2 ? 1 - (a / st_n) % 2 : t[1];
-        int c[6] = {st_n == 2 ? a % 2 : t[0], pr, ch_n == 2 ? ((a / (st_n * pr_n)) % 2 ? 32 : 8) : t[2], t[3], t[4],
-                    SB.precision == 4 && pr};
+        int c[7] = {st_n == 2 ? a % 2 : t[0], pr, ch_n == 2 ? ((a / (st_n * pr_n)) % 2 ? 32 : 8) : t[2], t[3], t[4],
+                    SB.precision == 4 && pr, 0};
         tune_apply(c);
         float im = 3.4e38f, pm = 3.4e38f;
         for (int r = 0; r < 2; r++) {
@@ -576,7 +594,7 @@ static int tune(const char *who)
     }
     if (cfg.blocks_per_sm < 0) {
         for (int bps = 3; bps >= 2; bps--) {
-            int c[6] = {best[0], best[1], best[2], bps, bps, best_i[1]};
+            int c[7] = {best[0], best[1], best[2], bps, bps, best_i[1], 0};
             tune_apply(c);
             float im = 3.4e38f, pm = 3.4e38f;
             for (int r = 0; r < 2; r++) {
@@ -592,6 +610,28 @@ static int tune(const char *who)
     }
     best[4] = best_i[0];
     best[5] = best_i[1];
+    if (tiles) {
+        if (fk_slabplan_tiles(&SB.plan, SB.precision, conv, who)) return 1;
+        const int cap = SB.plan.have_tiles ? fk3d_tile_capacity(SB.precision, SB.plan.dev.max_nz, conv) : 0;
+        if (cap > 0 && SB.plan.work_tiles[SB.plan.nwork] <= TILE_LAUNCHES * cap) {
+            int c[7];
+            memcpy(c, best, sizeof(c));
+            c[6] = 1;
+            tune_apply(c);
+            float m = 3.4e38f;
+            for (int r = 0; r < 2; r++) {
+                float i1, p1;
+                if (fk_check(tune_time(&i1, &p1), who)) return 1;
+                m = i1 + p1 < m ? i1 + p1 : m;
+                SB.tune_runs++;
+            }
+            if (m < best_init + best_pass) {
+                best[6] = 1;
+                best_init = 0.0f;
+                best_pass = m;
+            }
+        }
+    }
     tune_apply(best);
     SB.tune_ms[0] = best_init;
     SB.tune_ms[1] = best_pass;

@@ -87,9 +87,28 @@ typedef struct {
     const int *tasks_init;
     int ntask_init_sweep;
     int *done_t;                   /* nwork */
+    /* tile schedule (tile3d.cu), where use_tiles: every work item's tiles
+     * {work, bx | by << 16}, its first one, the edge words of a launch and
+     * their launch count (device); work_tiles[w]: tiles before work item w (host,
+     * nwork + 1) */
+    int use_tiles;
+    const int *tiles, *tile0;
+    unsigned long long *tile_edge;
+    unsigned *tile_epoch;
+    const int *work_tiles;
 } fk_slabs3d_t;
 
 #define FK_SLAB_Y 4
+
+/* Tile schedule: tiles of a grid; tiles of grids up to max_nz deep that are
+ * resident at once (0: none); bytes of edge words for ntile of them; the
+ * sweeps of a solve (called by fk3d_solve_slabs). */
+int fk3d_tiles(int nx, int ny);
+int fk3d_tile_capacity(int precision, int max_nz, int converge);
+size_t fk3d_tile_edge_bytes(int precision, int ntile, int max_nz);
+int fk3d_sweep_tiles(int precision, const fk_grid3d_t *grids, const fk_work3d_t *work, int nwork,
+                     const fk_slabs3d_t *plan, double eps, int npass, int converge, double conv_tol,
+                     cudaStream_t stream);
 
 /* Slab-pipelined solve of every work item: field initialisation, 8
  * initialisation sweeps, then nsweep passes of 8 sweeps (or, when conv_tol

@@ -1371,6 +1371,15 @@ inline int launch_rows(const fk_grid3d_t *grids, const fk_work3d_t *work, int nw
     P.s_end = 8;
     P.ticket = pl->tickets;
     if (fk3tw::g_slab_events) cudaEventRecord(fk3tw::g_slab_events[0], st);
+    if (pl->use_tiles) { /* every sweep in the tile schedule's launch */
+        if (fk3tw::g_slab_events) cudaEventRecord(fk3tw::g_slab_events[1], st);
+        const int rt = fk3d_sweep_tiles((int)sizeof(R), grids, work, nwork, pl, eps, npass, converge, conv_tol, st);
+        if (rt) return rt;
+        if (fk3tw::g_slab_events) cudaEventRecord(fk3tw::g_slab_events[2], st);
+        fk3tw::finalize_kernel<<<(nwork + 127) / 128, 128, 0, st>>>(nwork, npr, converge, npass, pl->resid,
+                                                                     pl->conv_pass, pl->error, results);
+        return (int)cudaGetLastError();
+    }
     /* initialisation with one source per thread: the turned-axes tasks ahead
      * of the slab tasks; their rings hold a y walk, so they are sized for
      * the deepest or widest grid */

@@ -13,6 +13,9 @@
 void fk_slabplan_free(fk_slabplan_t *pl)
 {
     fk_dfree(pl->mem);
+    fk_dfree(pl->tile_mem);
+    free(pl->nxy);
+    free(pl->work_tiles);
     memset(pl, 0, sizeof(*pl));
 }
 
@@ -99,13 +102,19 @@ int fk_slabplan_build(fk_slabplan_t *pl, int nwork, const int *nx, const int *ny
     if (!e) e = fk_check((int)fk_h2d(m + off_pairs, pairs, sizeof(int) * 2 * (size_t)npair), who);
     if (!e) e = fk_check((int)fk_h2d(m + off_t2, tasks2, sizeof(int) * 2 * (size_t)ntask2), who);
     if (!e) e = fk_check((int)fk_h2d(m + off_ti, tasks_i, sizeof(int) * 2 * (size_t)ntask_i), who);
+    int *nxy = (int *)malloc(sizeof(int) * 2 * (size_t)nwork);
+    for (int w = 0; nxy && w < nwork; w++) {
+        nxy[2 * w] = nx[w];
+        nxy[2 * w + 1] = ny[w];
+    }
+    pl->nxy = nxy;
     free(tasks_i);
     free(tasks);
     free(tasks2);
     free(pairs);
     free(base);
     free(nsl);
-    if (e) { fk_dfree(m); return 1; }
+    if (e || !nxy) { fk_dfree(m); free(nxy); pl->nxy = NULL; return 1; }
     pl->mem = m;
     pl->nwork = nwork;
     pl->npass = np;
@@ -130,5 +139,63 @@ int fk_slabplan_build(fk_slabplan_t *pl, int nwork, const int *nx, const int *ny
     pl->dev.tasks_init = (const int *)(m + off_ti);
     pl->dev.ntask_init_sweep = (int)ntask_i;
     pl->dev.done_t = (int *)(m + off_dt);
+    return 0;
+}
+
+int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who)
+{
+    const int key = 2 * precision + (converge != 0);
+    if (pl->work_tiles && pl->tile_key == key) return 0;
+    fk_dfree(pl->tile_mem);
+    free(pl->work_tiles);
+    pl->tile_mem = NULL;
+    pl->work_tiles = NULL;
+    pl->have_tiles = false;
+    pl->tile_key = key;
+    const int n = pl->nwork, nz = pl->dev.max_nz;
+    const int cap = fk3d_tile_capacity(precision, nz, converge);
+    int *wt = (int *)malloc(sizeof(int) * ((size_t)n + 1));
+    if (!wt) return 1;
+    long total = 0;
+    bool fit = cap > 0;
+    for (int w = 0; w < n; w++) {
+        const int k = fk3d_tiles(pl->nxy[2 * w], pl->nxy[2 * w + 1]);
+        wt[w] = (int)total;
+        fit = fit && k <= cap;
+        total += k;
+        if (total > (1L << 28)) fit = false;
+        if (!fit) break;
+    }
+    pl->work_tiles = wt;
+    if (!fit) return 0;
+    wt[n] = (int)total;
+    int *t = (int *)malloc(sizeof(int) * 2 * (size_t)total);
+    long k = 0;
+    for (int w = 0; t && w < n; w++) {
+        /* by rows of tiles: tile by ntx + bx of its work item */
+        const int k0 = wt[w], nk = wt[w + 1] - k0, ntx = (pl->nxy[2 * w] + 15) / 16;
+        for (int i = 0; i < nk; i++) {
+            t[2 * k] = w;
+            t[2 * k + 1] = i % ntx | (i / ntx) << 16;
+            k++;
+        }
+    }
+    const int most = total < cap ? (int)total : cap;   /* tiles of one launch */
+    const size_t off_0 = al(sizeof(int) * 2 * (size_t)total), off_e = off_0 + al(sizeof(int) * (size_t)n);
+    const size_t off_w = off_e + 256, bytes = off_w + fk3d_tile_edge_bytes(precision, most, nz);
+    char *m = t ? (char *)fk_dalloc(bytes, who) : NULL;
+    int e = m ? 0 : 1;
+    if (!e) e = fk_check((int)fk_h2d(m, t, sizeof(int) * 2 * (size_t)total), who);
+    if (!e) e = fk_check((int)fk_h2d(m + off_0, wt, sizeof(int) * (size_t)n), who);
+    if (!e) e = fk_check((int)fk_zero(m + off_e, bytes - off_e), who);
+    free(t);
+    if (e) { fk_dfree(m); return 1; }
+    pl->tile_mem = m;
+    pl->dev.tiles = (const int *)m;
+    pl->dev.tile0 = (const int *)(m + off_0);
+    pl->dev.tile_epoch = (unsigned *)(m + off_e);
+    pl->dev.tile_edge = (unsigned long long *)(m + off_w);
+    pl->dev.work_tiles = wt;
+    pl->have_tiles = true;
     return 0;
 }

@@ -2,12 +2,18 @@
 #ifndef FTEIK_SLABPLAN_H
 #define FTEIK_SLABPLAN_H
 #include "fteik_dev.h"
+#include <stdbool.h>
 
 typedef struct {
     fk_slabs3d_t dev; /* device pointers passed to fk3d_solve_slabs */
     void *mem;        /* the one device allocation behind them */
     int nwork, npass;
     const int *pairs_all; /* the source pairs (dev.pairs is this or NULL) */
+    int *nxy;             /* host [2 nwork]: nx, ny of every work item */
+    int *work_tiles;      /* host [nwork + 1] (dev.work_tiles) */
+    void *tile_mem;       /* device allocation of the tile schedule */
+    bool have_tiles;
+    int tile_key;         /* precision and convergence they were prepared for */
 } fk_slabplan_t;
 
 /* Build the plan for nwork work items with the given grid sizes and grid
@@ -18,4 +24,9 @@ typedef struct {
 int fk_slabplan_build(fk_slabplan_t *pl, int nwork, const int *nx, const int *ny, const int *nz,
                       const int *gid, int npass, int pairing, const char *who);
 void fk_slabplan_free(fk_slabplan_t *pl);
+/* Prepare the tile schedule of a built plan (once for a precision and
+ * convergence setting); have_tiles tells whether
+ * every work item's tiles fit the chip at once.  Returns 0 unless memory ran
+ * out. */
+int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who);
 #endif

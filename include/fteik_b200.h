@@ -389,7 +389,10 @@ void fteik_b200_batch3d_getTravelTimes64f(int igrid, int nval, double ttr[],
  * FTEIK_B200_TUNE_CACHE names a file, appended to that file for later
  * processes.  initMs / passMs: the chosen kernels' times during the search
  * (0 when nothing was searched), tuneRuns the candidate solves it ran (0 on
- * a cache hit).  No counterpart in the reference. */
+ * a cache hit).  With all four knobs left to the library, a work list whose
+ * tiles fit the chip may run as one kernel over tiles instead (tile3d.cu; the
+ * knobs then have no effect): initMs is 0 and passMs that kernel's time.  No
+ * counterpart in the reference. */
 void fteik_b200_batch3d_getSlabConfig(int *staged, int *pairs, int *progress, int *blocksPerSM,
                                       int *initBlocksPerSM, int *initPairs, float *initMs, float *passMs,
                                       int *tuneRuns, int *ierr);
