@@ -249,7 +249,7 @@ int fk_locate_l1_exact(int ngrd, int ldgrd, int ntf, const float *tables, int ne
 #define FK_TC_TOPK 4
 size_t fk_locate_tc_table_bytes(int ngrd);
 size_t fk_locate_tc_event_bytes(int nev);
-int fk_locate_tc_npart(int nev, int ngrd);
+int fk_locate_tc_npart(int nev, int ngrd, int few);   /* few: FK_TC_TOPK runs of an event are enough */
 int fk_locate_tc_pack_tables(int ngrd, int ldgrd, int ntf, const float *tables, void *bpack,
                              cudaStream_t s);
 int fk_locate_tc(int ngrd, int ldgrd, int ntf, const float *tables, const void *bpack,
@@ -260,9 +260,9 @@ int fk_locate_tc(int ngrd, int ldgrd, int ntf, const float *tables, const void *
 /* Pruned search: coarse runs (cand_* from fk_locate_tc on the coarse
  * surrogate tables [ntf][ldc], coarse node c = cz + ncz (cx + ncx cy) owning
  * the fine block [bz cz, bz cz + bz) x [bx cx, ..) x [by cy, ..)) -> the k best
- * coarse nodes (rc runs examined, rc <= 4, k <= 32) -> FP64 misfit on the
- * exact tables (block-major copy, fk_locate_block_tables) at every fine
- * node of their blocks, then a
+ * coarse nodes (rc runs examined, rc <= 4, k <= 32) -> misfit on the exact
+ * tables (block-major copy, fk_locate_block_tables) at every fine node of
+ * their blocks, in FP64 wherever FP32 cannot rule a node out, then a
  * descent over neighbouring blocks.  flag[e]: 0xFF when the event needs the
  * exhaustive search, else the number of blocks examined. */
 int fk_locate_prune(int nev, int npart, int rc, int k, int nz, int nx, int ny, int bz, int bx, int by,
@@ -271,7 +271,8 @@ int fk_locate_prune(int nev, int npart, int rc, int k, int nz, int nx, int ny, i
                     const float *cand_v, const int *cand_i, int *out_idx, double *out_t0,
                     double *out_obj, unsigned char *flag, cudaStream_t s);
 /* Block-major copy of tables [ntf][ldgrd] for fk_locate_prune's fine
- * stage: out [nblocks][ntf][bz bx by] (ncz ncx ncy blocks, z fastest). */
+ * stage: out [nblocks][ntf][bz bx by, rounded up to 4] (ncz ncx ncy blocks, z
+ * fastest). */
 int fk_locate_block_tables(int nz, int nx, int ny, int bz, int bx, int by, int ntf, int ldgrd,
                            const float *tables, float *out, cudaStream_t s);
 

@@ -405,7 +405,7 @@ static int ensure_tc(int n, int npart)
  * go through the exact search.  t0 excludes tepoch. */
 static int locate_range_tc(int e0, int n, int *idx, double *t0, double *obj)
 {
-    const int npart = fk_locate_tc_npart(n, SL.ngrd);
+    const int npart = fk_locate_tc_npart(n, SL.ngrd, 0);
     if (pack_tables() || upload_obs64() || ensure_tc(n, npart)) return 1;
     cudaStream_t s = fk_stream();
     int e = (int)cudaMemsetAsync(SL.err_dev, 0, sizeof(int), s);
@@ -721,8 +721,8 @@ void fteik_b200_locate_buildSurrogate(int bz, int bx, int by, int *ierr)
         if (!e) e = fk_mlp_coarse_store(r0, m, SP.ngrd_c, SP.ldc, tau, dist, SP.coarse, s);
     }
     if (!e) e = fk_locate_tc_pack_tables(SP.ngrd_c, SP.ldc, SL.ntf, SP.coarse, SP.bpack_c, s);
-    /* node-major block copy: each node's tables padded to a multiple of 4 */
-    const size_t nfine = (size_t)SP.ngrd_c * (size_t)((SL.ntf + 3) & ~3) * (size_t)(bz * bx * by);
+    /* block copy: a station's nodes of a block padded to a multiple of 4 */
+    const size_t nfine = (size_t)SP.ngrd_c * (size_t)SL.ntf * (size_t)((bz * bx * by + 3) & ~3);
     if (nfine != SP.fine_cap) {   /* a rebuild of the same blocks reuses the copy's memory */
         fk_dfree(SP.fine_blk);
         SP.fine_blk = (float *)fk_dalloc(sizeof(float) * nfine, who);
@@ -799,7 +799,7 @@ static int locate_tc_subset(const int *evs, int m, int *idx, double *t0, double 
         memcpy(hw + i * nt, SL.w64 + (size_t)evs[i] * nt, sizeof(double) * nt);
         he[i] = 1;
     }
-    const int npart = fk_locate_tc_npart(m, SL.ngrd);
+    const int npart = fk_locate_tc_npart(m, SL.ngrd, 0);
     int e = pack_tables() || ensure_tc(m, npart);
     cudaStream_t s = fk_stream();
     int kerr = 0;
@@ -835,7 +835,7 @@ static int locate_range_pruned(int e0, int n, int *idx, double *t0, double *obj)
         SP.blk_shape[1] = SP.bx;
         SP.blk_shape[2] = SP.by;
     }
-    const int npart = fk_locate_tc_npart(n, SP.ngrd_c);
+    const int npart = fk_locate_tc_npart(n, SP.ngrd_c, 1);   /* rc <= 4 runs are taken */
     if (upload_obs64() || ensure_tc(n, npart)) return 1;
     if (n > SP.flag_cap) {
         fk_dfree(SP.flag_dev);

@@ -503,32 +503,41 @@ __global__ void pack_tables_kernel(int ngrd, int ldgrd, int ntf, int ntile,
     *reinterpret_cast<uint4 *>(xt + xoff(r, 8)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-/* One thread per event row slot: -2 (o - mean o), split.  Rows of
- * ineligible or padding events are zero (their scores are not used). */
+/* Eight lanes per event row slot, one 8-station chunk each: -2 (o - mean o),
+ * split.  Rows of ineligible or padding events are zero (their scores are not
+ * used).  The mean's sum keeps the station order (one lane's additions), as a
+ * changed last bit could change a rounding to BF16. */
 __global__ void pack_events_kernel(int nev, int nrows, int ntf, const double *__restrict__ obs,
                                    const unsigned char *__restrict__ elig, uint8_t *__restrict__ apack)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double s_o[16][BK + 1];
+    const int e0 = blockIdx.x * 16;
+    for (int t = threadIdx.x; t < 16 * BK; t += 128) {
+        const int r = t / BK, k = t % BK, e = e0 + r;
+        s_o[r][k] = (e < nev && k < ntf) ? obs[(size_t)e * ntf + k] : 0.0;
+    }
+    __syncthreads();
+    const int rr = threadIdx.x >> 3, c = threadIdx.x & 7;
+    const int e = e0 + rr;
     if (e >= nrows) return;
     const int tile = e / BM, r = e % BM;
     uint8_t *hi = apack + (size_t)tile * PAIR_BYTES, *lo = hi + TILE_BYTES;
     const bool use = e < nev && elig[e];
     double mean = 0.0;
     if (use) {
-        for (int i = 0; i < ntf; ++i) mean += obs[(size_t)e * ntf + i];
+        for (int i = 0; i < ntf; ++i) mean += s_o[rr][i];
         mean /= (double)ntf;
     }
-    for (int c = 0; c < BK / 8; ++c) {
-        __align__(16) __nv_bfloat16 vh[8], vl[8];
-        for (int j = 0; j < 8; ++j) {
-            const int k = c * 8 + j;
-            const double d = (use && k < ntf) ? -2.0 * (obs[(size_t)e * ntf + k] - mean) : 0.0;
-            split_bf16(d, vh[j], vl[j]);
-        }
-        const uint32_t off = swz(r, c * 8);
-        *reinterpret_cast<uint4 *>(hi + off) = *reinterpret_cast<const uint4 *>(vh);
-        *reinterpret_cast<uint4 *>(lo + off) = *reinterpret_cast<const uint4 *>(vl);
+    __align__(16) __nv_bfloat16 vh[8], vl[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int k = c * 8 + j;
+        const double d = (use && k < ntf) ? -2.0 * (s_o[rr][k] - mean) : 0.0;
+        split_bf16(d, vh[j], vl[j]);
     }
+    const uint32_t off = swz(r, c * 8);
+    *reinterpret_cast<uint4 *>(hi + off) = *reinterpret_cast<const uint4 *>(vh);
+    *reinterpret_cast<uint4 *>(lo + off) = *reinterpret_cast<const uint4 *>(vl);
 }
 
 /* ---- FP64 re-score -------------------------------------------------------- */
@@ -668,52 +677,17 @@ __global__ void rescore_kernel(int nev, int npart, int ngrd, int ntf, int ldgrd,
 }
 
 
-/* a node's stations rounded up to 4 in the node-major block copy */
-__host__ __device__ __forceinline__ int ntf_pad(int ntf) { return (ntf + 3) & ~3; }
+/* a block's nodes rounded up to 4 in the block copy */
+__host__ __device__ __forceinline__ int nb_pad(int nb) { return (nb + 3) & ~3; }
 
-/* misfit64 of NP nodes whose tables are 16-byte aligned runs (node-major
- * block copy): the same operations in the same station order as
- * misfit64_n, four stations per load; row[j] == nullptr skips node j. */
-template <int NP>
-__device__ __forceinline__ void misfit64_rows(const float *const (&row)[NP], const float *dummy, int ntf,
-                                              const double *o, const double *w, double sw, double sw2,
-                                              double (&ob)[NP], double (&t0)[NP])
+/* Rounding allowance of the FP32 misfit of the pruned search: with e = 2^-24,
+ * s2 = sum d^2 and O2 = sum o^2 of the n <= 64 shifted picks o = d + T, the
+ * computed s2 - (sum d)^2 / n is within e ((3 n + 16) s2 + 5 sqrt(s2 O2)) of
+ * the exact one (o rounded once, each d, product and sum once; |sum d| <=
+ * sqrt(n s2)).  A few percent are added for the bound's own rounding. */
+__device__ __forceinline__ float var_slack(float s2, float o2)
 {
-    double a[NP], b[NP], c[NP];
-    const float4 *r4[NP];
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        a[j] = b[j] = c[j] = 0.0;
-        r4[j] = reinterpret_cast<const float4 *>(row[j] ? row[j] : dummy);
-    }
-    const int nq = ntf_pad(ntf) / 4;
-#pragma unroll 4
-    for (int q = 0; q < nq; ++q) {
-        float4 v[NP];
-#pragma unroll
-        for (int j = 0; j < NP; ++j) v[j] = __ldg(r4[j] + q);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = 4 * q + u;
-            if (i < ntf) {
-                const double wi = w[i], oi = o[i];
-#pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    const float tv = u == 0 ? v[j].x : u == 1 ? v[j].y : u == 2 ? v[j].z : v[j].w;
-                    const double d = oi - (double)tv;
-                    const double w2d = wi * wi * d;
-                    a[j] += wi * d;
-                    b[j] += w2d;
-                    c[j] += w2d * d;
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        t0[j] = a[j] / sw;
-        ob[j] = row[j] ? 0.5 * (c[j] - 2.0 * t0[j] * b[j] + t0[j] * t0[j] * sw2) : 1.0e300;
-    }
+    return 1.25e-5f * s2 + 3.2e-7f * sqrtf(s2 * o2);
 }
 
 /* ---- pruned search (surrogate coarse lattice) ---------------------------- */
@@ -731,16 +705,28 @@ struct PruneGeom {
  *     tables; the K best coarse nodes kept;
  *  2. every fine node of the K coarse nodes' blocks (coarse node c owns the
  *     fine nodes f with floor(f / b) = c on every axis: bz bx by per block,
- *     bz bx by K in all) scored in FP64 on the exact tables, read from their
- *     node-major block copy (each node's tables one 16-byte aligned run,
- *     read four stations per load); the minimum
- *     returned (first index among equal misfits);
+ *     bz bx by K in all) scored on the exact tables, first in FP32 (an
+ *     event's picks share one weight, so the misfit is w^2 / 2 times the
+ *     residuals' sum of squares about their mean: three operations a
+ *     station); a node whose FP32 misfit could, within its rounding, still be
+ *     the minimum is scored in FP64, and the minimum of those is returned
+ *     (first index among equal misfits).  The picks are shifted by the best
+ *     coarse node's origin time, so the residuals, and with them the
+ *     rounding, are small.  The tables are read from their block copy,
+ *     [block][station][node]: half a warp reads a station's 64 nodes, four
+ *     to a lane, in one contiguous load.  Scoring every node in FP64 from a
+ *     node-major copy (one line per lane and load, a conversion per value)
+ *     took 0.54 ms for 10,000 events x 8.4 blocks, this
+ *     0.36 ms, stage 1 included, half of the time its reads of HBM take;
  *  3. while a node next to that minimum (26-neighbourhood) lies in a block
  *     not yet examined, that block is examined too (a descent over blocks on
  *     the exact misfit, 32 blocks at most); flag[e] = 1 when the limit stops
  *     it, and the caller searches the event exhaustively.
  * flag[e]: 0xFF for a fall-back event, else the number of blocks examined. */
-__global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int RC, int K, PruneGeom G,
+/* (a CTA per event: events differ in their blocks, 0.36 against 0.38 ms with 8) */
+constexpr int PRUNE_WARPS = 1;
+
+__global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kernel(int nev, int npart, int RC, int K, PruneGeom G,
                              const float *__restrict__ coarse, const float *__restrict__ fine,
                              const double *__restrict__ obs, const double *__restrict__ wts,
                              const unsigned char *__restrict__ elig, const float *__restrict__ cand_v,
@@ -748,8 +734,9 @@ __global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int R
                              double *__restrict__ out_t0, double *__restrict__ out_obj,
                              unsigned char *__restrict__ flag)
 {
-    __shared__ int s_sel[8][32];   /* examined coarse nodes per warp */
-    __shared__ double s_o[8][BK], s_w[8][BK];
+    __shared__ int s_sel[PRUNE_WARPS][32];   /* examined coarse nodes per warp */
+    __shared__ double s_o[PRUNE_WARPS][BK], s_w[PRUNE_WARPS][BK];
+    __shared__ float s_of[PRUNE_WARPS][BK];  /* shifted picks */
     const int wib = threadIdx.x >> 5;
     const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -798,12 +785,10 @@ __global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int R
         const long long c = (long long)mi * RUN + lane;
         if (c < ncoarse) { cg[r] = c; cidx[r] = (int)c; }
     }
-    {
-        double ct0[4];
-        misfit64_n<4>(coarse, (size_t)G.ldc, cg, G.ntf, o, w, sw, sw2, cval, ct0);
-    }
+    double ct0[4];
+    misfit64_n<4>(coarse, (size_t)G.ldc, cg, G.ntf, o, w, sw, sw2, cval, ct0);
     /* 1b. the K best coarse nodes */
-    double pvd = -1.0e300;
+    double pvd = -1.0e300, tref = 0.0;
     int pid = -1;
     int nsel = 0;
     for (int k = 0; k < K; ++k) {
@@ -826,40 +811,97 @@ __global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int R
         pid = mi;
         if (lane == 0) s_sel[wib][k] = mi;
         nsel = k + 1;
+        if (k == 0) {     /* the best coarse node's origin time */
+            bool own = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (cidx[r] == mi && cg[r] >= 0) { own = true; tref = ct0[r]; }
+            const unsigned who = __ballot_sync(0xffffffffu, own);
+            tref = __shfl_sync(0xffffffffu, tref, who ? __ffs(who) - 1 : 0);
+        }
     }
     __syncwarp();
     /* 2. fine nodes of the selected blocks */
-    const int nb = G.bz * G.bx * G.by, ntp = ntf_pad(G.ntf);
+    const int nb = G.bz * G.bx * G.by, nbp = nb_pad(nb);
+    float o2 = 0.0f;
+    for (int i = lane; i < BK; i += 32) {
+        const float v = i < G.ntf ? (float)(o[i] - tref) : 0.0f;
+        s_of[wib][i] = v;
+        o2 = fmaf(v, v, o2);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) o2 += __shfl_xor_sync(0xffffffffu, o2, s);
+    __syncwarp();
+    const float *of = s_of[wib];
+    const float inv_n = 1.0f / (float)G.ntf;
+    const double to_var = 2.0 / (w[0] * w[0]);    /* misfit -> sum of squares */
+    float ub = __int_as_float(0x7f800000);        /* above the best sum of squares so far */
+    /* a lane's two nodes in a block (past the block's end: outside the grid) */
+    int oz[2], ox[2], oy[2];
+    auto place = [&](int p0, int j) {
+        const int pn = p0 + 4 * (lane & 15) + 2 * (lane >> 4) + j;
+        oz[j] = pn < nb ? pn % G.bz : 1 << 29;
+        ox[j] = (pn / G.bz) % G.bx;
+        oy[j] = pn / (G.bz * G.bx);
+    };
+    place(0, 0);
+    place(0, 1);
     double best = 1.0e300, bt0 = 0.0;
     int bg = 0x7fffffff, bk = -1;
     auto scan_block = [&](int k) {
         const int c = s_sel[wib][k];
         const int cz = c % G.ncz, cx = (c / G.ncz) % G.ncx, cy = c / (G.ncz * G.ncx);
-        for (int p0 = lane; p0 < nb; p0 += 64) {
-            long long g2[2];
+        const float *const blk = fine + (size_t)c * G.ntf * nbp;
+        bool scored = false;
+        if (nb > 64) { place(0, 0); place(0, 1); }
+        for (int p0 = 0; p0 < nb; p0 += 64) {
+            const int pq = p0 + 4 * (lane & 15), half = lane >> 4;
+            float s1[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (pq < nbp) {
+                const float *src = blk + (size_t)half * nbp + pq;
+#pragma unroll 8
+                for (int i = half; i < G.ntf; i += 2, src += 2 * nbp) {
+                    const float4 t = __ldg(reinterpret_cast<const float4 *>(src));
+                    const float oi = of[i];
+                    const float d0 = oi - t.x, d1 = oi - t.y, d2 = oi - t.z, d3 = oi - t.w;
+                    s1[0] += d0; s1[1] += d1; s1[2] += d2; s1[3] += d3;
+                    s2[0] = fmaf(d0, d0, s2[0]); s2[1] = fmaf(d1, d1, s2[1]);
+                    s2[2] = fmaf(d2, d2, s2[2]); s2[3] = fmaf(d3, d3, s2[3]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 16);
+                s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 16);
+            }
+            /* each half keeps two of the four nodes */
+            float v[2], sl[2];
+            int g2[2];
+            float m = __int_as_float(0x7f800000);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int p = p0 + 32 * j;
-                const int fz = G.bz * cz + p % G.bz, fx = G.bx * cx + (p / G.bz) % G.bx,
-                          fy = G.by * cy + p / (G.bz * G.bx);
-                g2[j] = (p < nb && fz < G.nz && fx < G.nx && fy < G.ny)
-                            ? fz + (long long)G.nz * (fx + (long long)G.nx * fy) : -1;
+                const float a = half ? s1[2 + j] : s1[j], q = half ? s2[2 + j] : s2[j];
+                v[j] = q - a * a * inv_n;
+                sl[j] = var_slack(q, o2);
+                if (p0 > 0) place(p0, j);
+                const int fz = G.bz * cz + oz[j], fx = G.bx * cx + ox[j], fy = G.by * cy + oy[j];
+                g2[j] = (fz < G.nz && fx < G.nx && fy < G.ny)
+                            ? (int)(fz + (long long)G.nz * (fx + (long long)G.nx * fy)) : -1;
+                if (g2[j] >= 0) m = fminf(m, v[j] + sl[j]);
             }
-            /* each node's tables are one 16-byte aligned run in the node-major block copy */
-            long long q2[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) q2[j] = g2[j] >= 0 ? p0 + 32 * j : -1;
-            double ob[2], t0[2];
-            const float *rows[2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) rows[j] = q2[j] >= 0 ? fine + ((size_t)c * nb + q2[j]) * ntp : nullptr;
-            misfit64_rows<2>(rows, fine, G.ntf, o, w, sw, sw2, ob, t0);
+            for (int s = 16; s > 0; s >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, s));
+            m = fminf(m, ub);
 #pragma unroll
             for (int j = 0; j < 2; ++j)
-                if (g2[j] >= 0 && lex_lt_d(ob[j], (int)g2[j], best, bg)) {
-                    best = ob[j]; bg = (int)g2[j]; bt0 = t0[j]; bk = k;
+                if (g2[j] >= 0 && !(v[j] - sl[j] > m)) {   /* NaN: scored */
+                    double ob, t0;
+                    ob = misfit64(blk, (size_t)nbp, pq + 2 * half + j, G.ntf, o, w, sw, sw2, t0);
+                    if (lex_lt_d(ob, g2[j], best, bg)) { best = ob; bg = g2[j]; bt0 = t0; bk = k; }
+                    scored = true;
                 }
         }
+        if (!__any_sync(0xffffffffu, scored)) return;
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1) {
             const double ob = __shfl_xor_sync(0xffffffffu, best, s);
@@ -868,6 +910,7 @@ __global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int R
             const int ok = __shfl_xor_sync(0xffffffffu, bk, s);
             if (lex_lt_d(ob, og, best, bg)) { best = ob; bg = og; bt0 = ot; bk = ok; }
         }
+        ub = __double2float_ru(best * to_var * (1.0 + 1e-6));   /* misfit64's own rounding is far below */
     };
     for (int k = 0; k < nsel; ++k) scan_block(k);
     /* 3. while a neighbour of the minimum lies in a block not yet examined,
@@ -908,33 +951,26 @@ __global__ void __launch_bounds__(256, 3) prune_kernel(int nev, int npart, int R
     flag[e] = fb ? (unsigned char)0xFF : (unsigned char)nsel;
 }
 
-/* Block-major, node-major copy of the exact tables for the pruned search:
- * out[(c nb + p) ntp + i] = T_i(node p of block c), p = pz + bz (px + bx py),
- * ntp = ntf rounded up to 4 (a node's tables are one 16-byte aligned run);
- * padding and nodes outside the grid hold 0 (never read). */
+/* Block-major copy of the exact tables for the pruned search:
+ * out[(c ntf + i) nbp + p] = T_i(node p of block c), p = pz + bz (px + bx py),
+ * nbp = bz bx by rounded up to 4 (a station's nodes are 16-byte aligned);
+ * padding and nodes outside the grid hold 0 (never used). */
 __global__ void block_tables_kernel(int nz, int nx, int ny, int bz, int bx, int by, int ncz, int ncx, int ntf,
                                     int ldgrd, long long nblk, const float *__restrict__ tables,
                                     float *__restrict__ out)
 {
-    const int nb = bz * bx * by, ntp = ntf_pad(ntf);
+    const int nb = bz * bx * by, nbp = nb_pad(nb);
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= nblk * nb) return;
-    const long long c = t / nb;
-    const int p = (int)(t % nb);
+    if (t >= nblk * nbp) return;
+    const long long c = t / nbp;
+    const int p = (int)(t % nbp);
     const int cz = (int)(c % ncz), cx = (int)((c / ncz) % ncx), cy = (int)(c / ((long long)ncz * ncx));
     const int fz = bz * cz + p % bz, fx = bx * cx + (p / bz) % bx, fy = by * cy + p / (bz * bx);
-    const bool in = fz < nz && fx < nx && fy < ny;
+    const bool in = p < nb && fz < nz && fx < nx && fy < ny;
     const long long g = in ? fz + (long long)nz * (fx + (long long)nx * fy) : 0;
-    float4 *dst = reinterpret_cast<float4 *>(out + (size_t)t * ntp);
-    for (int q = 0; q < ntp / 4; ++q) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = 4 * q + u;
-            v[u] = (in && i < ntf) ? __ldg(tables + (size_t)i * ldgrd + g) : 0.0f;
-        }
-        dst[q] = make_float4(v[0], v[1], v[2], v[3]);
-    }
+    float *dst = out + (size_t)c * ntf * nbp + p;
+#pragma unroll 8
+    for (int i = 0; i < ntf; ++i) dst[(size_t)i * nbp] = in ? __ldg(tables + (size_t)i * ldgrd + g) : 0.0f;
 }
 
 } // namespace fktc
@@ -982,19 +1018,41 @@ static int pick_npart(int nmg, int ntile, int nsm)
     return best;
 }
 
+/* The same for a caller that takes at most TOPK runs of an event: however few
+ * partitions, each keeps its TOPK best, so the best TOPK of all are among them.
+ * The fewest waves that are nearly full: a work item's first loads and last
+ * epilogue do not overlap its products (10,000 events x 38,400 coarse points:
+ * 11 partitions of 27 tiles; with the packing 117 us against 145 with 37 of 8). */
+static int pick_npart_few(int nmg, int ntile, int nsm)
+{
+    int best = 1;
+    double best_eff = -1.0;
+    for (int waves = 1; waves <= 16; ++waves) {
+        int P = waves * nsm / nmg;
+        if (P > ntile) P = ntile;
+        if (P < 1) continue;
+        const long long items = (long long)P * nmg;
+        const long long slots = (items + nsm - 1) / nsm * nsm;
+        const double eff = (double)items / (double)slots;
+        if (eff > best_eff + 1e-9) { best_eff = eff; best = P; }
+        if (eff > 0.97 || P == ntile) break;
+    }
+    return best_eff < 0.0 ? 1 : best;
+}
+
 /* products of the ranking, 2 (the default) or 3 (l2_tc_kernel<NPROD>) */
 static int g_nprod = 2;
 extern "C" void fk_locate_tc_set_products(int n) { g_nprod = n == 2 ? 2 : 3; }
 extern "C" int fk_locate_tc_get_products(void) { return g_nprod; }
 
-extern "C" int fk_locate_tc_npart(int nev, int ngrd)
+extern "C" int fk_locate_tc_npart(int nev, int ngrd, int few)
 {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int nmg = (nev + 2 * BM - 1) / (2 * BM);
     const int ntile = (ngrd + BN - 1) / BN;
-    return pick_npart(nmg, ntile, nsm);
+    return few ? pick_npart_few(nmg, ntile, nsm) : pick_npart(nmg, ntile, nsm);
 }
 
 extern "C" int fk_locate_tc(int ngrd, int ldgrd, int ntf, const float *tables, const void *bpack,
@@ -1008,7 +1066,7 @@ extern "C" int fk_locate_tc(int ngrd, int ldgrd, int ntf, const float *tables, c
     const int nmg = (nev + 2 * BM - 1) / (2 * BM);
     const int ntile = (ngrd + BN - 1) / BN;
     if (npart > ntile) return (int)cudaErrorInvalidValue;
-    pack_events_kernel<<<(nmg * 2 * BM + 127) / 128, 128, 0, s>>>(nev, nmg * 2 * BM, ntf, obs, elig,
+    pack_events_kernel<<<(nmg * 2 * BM + 15) / 16, 128, 0, s>>>(nev, nmg * 2 * BM, ntf, obs, elig,
                                                                   (uint8_t *)apack);
     static int attr_done = 0;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1068,7 +1126,7 @@ extern "C" int fk_locate_prune(int nev, int npart, int rc, int k, int nz, int nx
     G.ncx = (nx + bx - 1) / bx;
     G.ncy = (ny + by - 1) / by;
     G.ldgrd = ldgrd; G.ldc = ldc; G.ntf = ntf;
-    prune_kernel<<<(nev * 32 + 255) / 256, 256, 0, s>>>(nev, npart, rc, k, G, coarse, fine, obs, wts, elig,
+    prune_kernel<<<(nev + PRUNE_WARPS - 1) / PRUNE_WARPS, 32 * PRUNE_WARPS, 0, s>>>(nev, npart, rc, k, G, coarse, fine, obs, wts, elig,
                                                         cand_v, cand_i, out_idx, out_t0, out_obj, flag);
     return (int)cudaGetLastError();
 }
@@ -1078,7 +1136,7 @@ extern "C" int fk_locate_block_tables(int nz, int nx, int ny, int bz, int bx, in
 {
     const int ncz = (nz + bz - 1) / bz, ncx = (nx + bx - 1) / bx, ncy = (ny + by - 1) / by;
     const long long nblk = (long long)ncz * ncx * ncy;
-    const long long n = nblk * bz * bx * by;
+    const long long n = nblk * nb_pad(bz * bx * by);
     block_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(nz, nx, ny, bz, bx, by, ncz, ncx, ntf, ldgrd,
                                                                     nblk, tables, out);
     return (int)cudaGetLastError();
