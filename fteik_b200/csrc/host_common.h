@@ -59,6 +59,7 @@ typedef struct {
     double *slow;          /* host FP64, natural cell order */
     void *slow_dev32;      /* device FP32 padded */
     void *slow_dev64;      /* device FP64 padded */
+    double *slow_tmp;      /* device [ncell]: the slowness before padding */
     float *slowz_dev;      /* device FP32 node-indexed copies (3D; fk_grid3d_t.slowz) */
     bool dev32_ok, dev64_ok, devz_ok;
 } fk_model_t;

@@ -32,6 +32,7 @@ void fteik_model_free(void)
     free(fk_model.slow);
     fk_dfree(fk_model.slow_dev32);
     fk_dfree(fk_model.slow_dev64);
+    fk_dfree(fk_model.slow_tmp);
     fk_dfree(fk_model.slowz_dev);
     memset(&fk_model, 0, sizeof(fk_model));
     fk_model.lis3d = true;
@@ -64,6 +65,7 @@ void fteik_model_setGridSize(bool lis3d, int nz, int nx, int ny, int *ierr)
     fk_model.slow = (double *)calloc((size_t)fk_model.ncell, sizeof(double));
     fk_dfree(fk_model.slow_dev32); fk_model.slow_dev32 = NULL;
     fk_dfree(fk_model.slow_dev64); fk_model.slow_dev64 = NULL;
+    fk_dfree(fk_model.slow_tmp); fk_model.slow_tmp = NULL;
     fk_dfree(fk_model.slowz_dev); fk_model.slowz_dev = NULL;
     fk_model_invalidate_dev();
     fk_model.have_model = false;
@@ -155,8 +157,29 @@ int fteik_model_velGrid2indexF(int i, int j, int k, int nzm1, int nzm1_nxm1)
 }
 
 /* --------------------------------------------------------- velocities -- */
+/* Plain loops, vectorised where the host can (2 million cells: 4.4 ms with
+ * the scalar ones). */
+#if defined(__x86_64__) && defined(__GNUC__) && !defined(__clang__)
+#define FK_VECTOR __attribute__((optimize("O3"), target_clones("avx2", "default")))
+#else
+#define FK_VECTOR
+#endif
+
+FK_VECTOR static long count_not_positive(const double *v, long n)
+{
+    long bad = 0;
+    for (long i = 0; i < n; i++) bad += v[i] <= 0.0;
+    return bad;
+}
+
+FK_VECTOR static void invert(const double *v, double *s, long n)
+{
+    for (long i = 0; i < n; i++) s[i] = 1.0 / v[i];
+}
+
 static int check_positive(const double *v, long n, const char *who)
 {
+    if (v[0] > 0.0 && count_not_positive(v, n) == 0) return 0;
     double vmin = v[0];
     for (long i = 1; i < n; i++) if (v[i] < vmin) vmin = v[i];
     if (!(vmin > 0.0)) {
@@ -177,7 +200,7 @@ void fteik_model_setVelocityModel64f(int nv, const double vel[], int *ierr)
         return;
     }
     if (check_positive(vel, nv, "fteik_model_setVelocityModel64f")) { *ierr = 1; return; }
-    for (int i = 0; i < nv; i++) fk_model.slow[i] = 1.0 / vel[i];
+    invert(vel, fk_model.slow, nv);
     fk_model_invalidate_dev();
     fk_model.have_model = true;
 }
@@ -274,7 +297,7 @@ void fteik_model_setCellVelocityModel64f(int nc, int order, const double vel[], 
     } else {
         if (order != FTEIK_NATURAL_ORDERING && fk_model.verbose > 0)
             fprintf(stdout, "fteik_model_setCellVelocityModel64f: Defaulting to natural order\n");
-        for (int i = 0; i < ncell; i++) fk_model.slow[i] = 1.0 / vel[i];
+        invert(vel, fk_model.slow, ncell);
     }
     fk_model_invalidate_dev();
     fk_model.have_model = true;
@@ -361,14 +384,15 @@ const void *fk_model_slow_dev(int precision)
         *slot = fk_dalloc(nelem * (size_t)precision, "fteik_model");
         if (!*slot) return NULL;
     }
-    double *tmp = (double *)fk_dalloc(sizeof(double) * (size_t)fk_model.ncell, "fteik_model");
+    /* the staging buffer stays with the grid: a free waits for the device */
+    if (!fk_model.slow_tmp) fk_model.slow_tmp = (double *)fk_dalloc(sizeof(double) * (size_t)fk_model.ncell, "fteik_model");
+    double *tmp = fk_model.slow_tmp;
     if (!tmp) return NULL;
     int e = (int)cudaMemsetAsync(*slot, 0, nelem * (size_t)precision, fk_stream());
     if (!e) e = (int)cudaMemcpyAsync(tmp, fk_model.slow, sizeof(double) * (size_t)fk_model.ncell,
                                     cudaMemcpyHostToDevice, fk_stream());
     if (!e) e = fk_pack_slowness(precision, fk_model.lis3d, nz, nx, ny, zcp, tmp, *slot, fk_stream());
     if (!e) e = (int)cudaStreamSynchronize(fk_stream());
-    fk_dfree(tmp);
     if (fk_check(e, "fteik_model: slowness upload")) return NULL;
     *ok = true;
     return *slot;

@@ -49,6 +49,9 @@ static struct {
     int tc_cap;
     int *err_dev;
     float *dbg_dev;
+    char *pin;               /* page-locked host buffer for results on their way */
+    size_t pin_cap;
+    int lo, hi, lo64, hi64;  /* events set since the last upload (dirty, dirty64) */
 } SL;
 
 /* Surrogate-pruned search state: grid geometry of the tables, station
@@ -104,6 +107,7 @@ void locate_finalize(void)
     fk_dfree(SL.apack); fk_dfree(SL.cand_v); fk_dfree(SL.cand_i);
     fk_dfree(SL.tc_idx); fk_dfree(SL.tc_t0); fk_dfree(SL.tc_obj); fk_dfree(SL.err_dev);
     fk_dfree(SL.dbg_dev);
+    if (SL.pin) cudaFreeHost(SL.pin);
     memset(&SL, 0, sizeof(SL));
 }
 
@@ -167,6 +171,8 @@ void locate_initialize(int nEvents, int ntf, int ngrd, int *ierr)
     SL.init = true;
     SL.dirty = true;
     SL.dirty64 = true;
+    SL.lo = SL.lo64 = 0;     /* every event, once */
+    SL.hi = SL.hi64 = nEvents;
     SL.tables_dirty = true;
     SL.table_gen++;
     SL.rescore = 8;
@@ -284,6 +290,10 @@ void locate_setObservation64f(int evnmbr, int nttimes, bool lhaveOT, double t0,
     SL.l1ok[evnmbr - 1] = (l1 && wref > 0.0) ? 1 : 0;
     SL.dirty = true;
     SL.dirty64 = true;
+    if (evnmbr - 1 < SL.lo) SL.lo = evnmbr - 1;
+    if (evnmbr > SL.hi) SL.hi = evnmbr;
+    if (evnmbr - 1 < SL.lo64) SL.lo64 = evnmbr - 1;
+    if (evnmbr > SL.hi64) SL.hi64 = evnmbr;
 }
 
 void locate_setObservation64fC(int evnmbr, int nttimes, bool lhaveOT, double t0,
@@ -295,6 +305,38 @@ void locate_setObservation64fC(int evnmbr, int nttimes, bool lhaveOT, double t0,
     for (int i = 0; i < nttimes; i++) f[i] = obs2tf[i] + 1;
     locate_setObservation64f(evnmbr + 1, nttimes, lhaveOT, t0, f, pickTimes, wts, ierr);
     free(f);
+}
+
+/* Device results src[k] of bytes[k] to the caller's arrays dst[k], and the
+ * stream drained: through one page-locked buffer up to PIN_MAX (a copy into
+ * pageable memory waits by itself, 10 us each), else directly. */
+#define PIN_MAX ((size_t)4 << 20)
+
+static int fetch_results(int parts, void *const dst[], const void *const src[], const size_t bytes[], cudaStream_t s)
+{
+    size_t total = 0;
+    for (int k = 0; k < parts; k++) total += (bytes[k] + 15) & ~(size_t)15;
+    if (total <= PIN_MAX && total > SL.pin_cap) {
+        if (SL.pin) cudaFreeHost(SL.pin);
+        void *p = NULL;
+        SL.pin = cudaHostAlloc(&p, total, cudaHostAllocDefault) == cudaSuccess ? (char *)p : NULL;
+        SL.pin_cap = SL.pin ? total : 0;
+        if (!SL.pin) (void)cudaGetLastError();
+    }
+    const bool staged = total <= SL.pin_cap;
+    int e = 0;
+    size_t off = 0;
+    for (int k = 0; k < parts && !e; k++) {
+        e = (int)cudaMemcpyAsync(staged ? (void *)(SL.pin + off) : dst[k], src[k], bytes[k], cudaMemcpyDeviceToHost, s);
+        off += (bytes[k] + 15) & ~(size_t)15;
+    }
+    if (!e) e = (int)cudaStreamSynchronize(s);
+    off = 0;
+    for (int k = 0; k < parts && !e && staged; k++) {
+        memcpy(dst[k], SL.pin + off, bytes[k]);
+        off += (bytes[k] + 15) & ~(size_t)15;
+    }
+    return e;
 }
 
 static int ensure_out(int n)
@@ -314,11 +356,13 @@ static int upload_obs(void)
 {
     if (!SL.dirty) return 0;
     cudaStream_t s = fk_stream();
-    size_t n = (size_t)SL.nev * SL.ntf;
-    int e = (int)cudaMemcpyAsync(SL.obs_dev, SL.obs, sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    if (!e) e = (int)cudaMemcpyAsync(SL.wts_dev, SL.wts, sizeof(float) * n, cudaMemcpyHostToDevice, s);
+    const size_t o = (size_t)SL.lo * SL.ntf, n = (size_t)(SL.hi - SL.lo) * SL.ntf;
+    int e = (int)cudaMemcpyAsync(SL.obs_dev + o, SL.obs + o, sizeof(float) * n, cudaMemcpyHostToDevice, s);
+    if (!e) e = (int)cudaMemcpyAsync(SL.wts_dev + o, SL.wts + o, sizeof(float) * n, cudaMemcpyHostToDevice, s);
     if (fk_check(e, "locate: observation upload")) return 1;
     SL.dirty = false;
+    SL.lo = SL.nev;
+    SL.hi = 0;
     return 0;
 }
 
@@ -330,10 +374,10 @@ static int locate_range(int e0, int n, int *idx, float *t0, float *obj)
     int e = fk_locate_l2_exact(SL.ngrd, SL.ldgrd, SL.ntf, SL.tables, n,
                                SL.obs_dev + (size_t)e0 * SL.ntf, SL.wts_dev + (size_t)e0 * SL.ntf,
                                SL.idx_dev, SL.t0_dev, SL.obj_dev, SL.scratch, SL.scratch_bytes, s);
-    if (!e) e = (int)cudaMemcpyAsync(idx, SL.idx_dev, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(t0, SL.t0_dev, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(obj, SL.obj_dev, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaStreamSynchronize(s);
+    if (!e)
+        e = fetch_results(3, (void *const[]){idx, t0, obj}, (const void *const[]){SL.idx_dev, SL.t0_dev, SL.obj_dev},
+                          (const size_t[]){sizeof(int) * (size_t)n, sizeof(float) * (size_t)n, sizeof(float) * (size_t)n},
+                          s);
     return fk_check(e, "locate");
 }
 
@@ -346,13 +390,20 @@ static int upload_obs64(void)
         SL.w64_dev = (double *)fk_dalloc(sizeof(double) * n, "locate");
         SL.elig_dev = (unsigned char *)fk_dalloc((size_t)SL.nev, "locate");
         if (!SL.obs64_dev || !SL.w64_dev || !SL.elig_dev) return 1;
+        SL.lo64 = 0;
+        SL.hi64 = SL.nev;
     }
     cudaStream_t s = fk_stream();
-    int e = (int)cudaMemcpyAsync(SL.obs64_dev, SL.obs64, sizeof(double) * n, cudaMemcpyHostToDevice, s);
-    if (!e) e = (int)cudaMemcpyAsync(SL.w64_dev, SL.w64, sizeof(double) * n, cudaMemcpyHostToDevice, s);
-    if (!e) e = (int)cudaMemcpyAsync(SL.elig_dev, SL.elig, (size_t)SL.nev, cudaMemcpyHostToDevice, s);
+    const size_t o = (size_t)SL.lo64 * SL.ntf, m = (size_t)(SL.hi64 - SL.lo64) * SL.ntf;
+    int e = (int)cudaMemcpyAsync(SL.obs64_dev + o, SL.obs64 + o, sizeof(double) * m, cudaMemcpyHostToDevice, s);
+    if (!e) e = (int)cudaMemcpyAsync(SL.w64_dev + o, SL.w64 + o, sizeof(double) * m, cudaMemcpyHostToDevice, s);
+    if (!e)
+        e = (int)cudaMemcpyAsync(SL.elig_dev + SL.lo64, SL.elig + SL.lo64, (size_t)(SL.hi64 - SL.lo64),
+                                 cudaMemcpyHostToDevice, s);
     if (fk_check(e, "locate: FP64 observation upload")) return 1;
     SL.dirty64 = false;
+    SL.lo64 = SL.nev;
+    SL.hi64 = 0;
     return 0;
 }
 
@@ -415,11 +466,11 @@ static int locate_range_tc(int e0, int n, int *idx, double *t0, double *obj)
                          SL.elig_dev + e0, SL.apack, npart, SL.cand_v, SL.cand_i, SL.rescore,
                          SL.tc_idx, SL.tc_t0, SL.tc_obj, SL.err_dev, SL.dbg_dev, s);
     int kerr = 0;
-    if (!e) e = (int)cudaMemcpyAsync(idx, SL.tc_idx, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(t0, SL.tc_t0, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(obj, SL.tc_obj, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(&kerr, SL.err_dev, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaStreamSynchronize(s);
+    if (!e)
+        e = fetch_results(4, (void *const[]){idx, t0, obj, &kerr},
+                          (const void *const[]){SL.tc_idx, SL.tc_t0, SL.tc_obj, SL.err_dev},
+                          (const size_t[]){sizeof(int) * (size_t)n, sizeof(double) * (size_t)n,
+                                           sizeof(double) * (size_t)n, sizeof(int)}, s);
     if (fk_check(e, "locate (tensor core)")) return 1;
     if (kerr) {
         FK_ERR("locate (tensor core): pipeline wait timed out (code %d)", kerr);
@@ -521,10 +572,10 @@ static int locate_range_l1(int e0, int n, int *idx, double *t0, double *obj)
     int e = fk_locate_l1_exact(SL.ngrd, SL.ldgrd, SL.ntf, SL.tables, n, SL.obs_dev + (size_t)e0 * SL.ntf,
                                SL.wts_dev + (size_t)e0 * SL.ntf, SL.obs64_dev + (size_t)e0 * SL.ntf,
                                SL.w64_dev + (size_t)e0 * SL.ntf, SL.l1_idx, SL.l1_t0, SL.l1_obj, SL.l1_best, s);
-    if (!e) e = (int)cudaMemcpyAsync(idx, SL.l1_idx, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(t0, SL.l1_t0, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(obj, SL.l1_obj, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaStreamSynchronize(s);
+    if (!e)
+        e = fetch_results(3, (void *const[]){idx, t0, obj}, (const void *const[]){SL.l1_idx, SL.l1_t0, SL.l1_obj},
+                          (const size_t[]){sizeof(int) * (size_t)n, sizeof(double) * (size_t)n,
+                                           sizeof(double) * (size_t)n}, s);
     return fk_check(e, "locate (L1)");
 }
 
@@ -861,13 +912,15 @@ static int locate_range_pruned(int e0, int n, int *idx, double *t0, double *obj)
                             SL.w64_dev + (size_t)e0 * SL.ntf, SL.elig_dev + e0, SL.cand_v, SL.cand_i,
                             SL.tc_idx, SL.tc_t0, SL.tc_obj, SP.flag_dev, s);
     if (!e && SP.timing) e = (int)cudaEventRecord(SP.ev[2], s);
-    if (!e) e = (int)cudaMemcpyAsync(idx, SL.tc_idx, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(t0, SL.tc_t0, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(obj, SL.tc_obj, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(flag, SP.flag_dev, (size_t)n, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(&kerr, SL.err_dev, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (!e && SP.timing) e = (int)cudaEventRecord(SP.ev[3], s);
-    if (!e) e = (int)cudaStreamSynchronize(s);
+    if (!e)
+        e = fetch_results(5, (void *const[]){idx, t0, obj, flag, &kerr},
+                          (const void *const[]){SL.tc_idx, SL.tc_t0, SL.tc_obj, SP.flag_dev, SL.err_dev},
+                          (const size_t[]){sizeof(int) * (size_t)n, sizeof(double) * (size_t)n,
+                                           sizeof(double) * (size_t)n, (size_t)n, sizeof(int)}, s);
+    if (!e && SP.timing) {
+        e = (int)cudaEventRecord(SP.ev[3], s);
+        if (!e) e = (int)cudaStreamSynchronize(s);
+    }
     if (!e && SP.timing)
         for (int k = 0; k < 3; k++) cudaEventElapsedTime(&SP.stage_ms[k], SP.ev[k], SP.ev[k + 1]);
     if (fk_check(e, "locate (surrogate-pruned)") || kerr) {

@@ -76,14 +76,16 @@ static struct {
     float *z[MLP_MAXL];                /* pre-activations */
     float *dz, *dtmp;                  /* backward scratch [cap][width] */
     double *loss_dev;
+    float *y;                          /* targets of a gradient call [cap] */
+    float *pin;                        /* page-locked host buffer [nparam + 2]: the gradient and loss on their way */
 } NN;
 
 static void mlp_free_buffers(void)
 {
     for (int l = 0; l <= MLP_MAXL; l++) { fk_dfree(NN.x[l]); NN.x[l] = NULL; }
     for (int l = 0; l < MLP_MAXL; l++) { fk_dfree(NN.z[l]); NN.z[l] = NULL; }
-    fk_dfree(NN.dz); fk_dfree(NN.dtmp);
-    NN.dz = NN.dtmp = NULL;
+    fk_dfree(NN.dz); fk_dfree(NN.dtmp); fk_dfree(NN.y);
+    NN.dz = NN.dtmp = NN.y = NULL;
     NN.cap = 0;
 }
 
@@ -98,6 +100,7 @@ void fteik_b200_mlp_finalize(void)
     g_wq = NULL;
     g_wq_cap = 0;
     fk_dfree(NN.w); fk_dfree(NN.g); fk_dfree(NN.m); fk_dfree(NN.v); fk_dfree(NN.wt); fk_dfree(NN.loss_dev);
+    if (NN.pin) cudaFreeHost(NN.pin);
     memset(&NN, 0, sizeof(NN));
 }
 
@@ -306,15 +309,25 @@ void fteik_b200_mlp_gradient(int n, const float x[], const float y[], double *lo
     if (!NN.init || n < 1) { FK_ERR("fteik_b200_mlp_gradient: not initialized or n < 1"); return; }
     if (ensure_batch(n)) return;
     cudaStream_t s = fk_stream();
-    float *ydev = (float *)fk_dalloc(sizeof(float) * (size_t)n, "mlp");
-    if (!ydev) return;
+    if (!NN.y) NN.y = (float *)fk_dalloc(sizeof(float) * (size_t)NN.cap, "mlp");
+    if (!NN.y) return;
+    if (!NN.pin) {   /* copies into it are queued; without it they go to pageable memory */
+        void *p = NULL;
+        if (cudaHostAlloc(&p, sizeof(float) * (NN.nparam + 4), cudaHostAllocDefault) == cudaSuccess) NN.pin = (float *)p;
+        else (void)cudaGetLastError();
+    }
+    const size_t gb = sizeof(float) * NN.nparam, lo = (NN.nparam + 1) & ~(size_t)1;   /* the loss on 8 bytes */
     int e = (int)cudaMemcpyAsync(NN.x[0], x, sizeof(float) * (size_t)n * MLP_IN, cudaMemcpyHostToDevice, s);
-    if (!e) e = (int)cudaMemcpyAsync(ydev, y, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, s);
-    if (!e) e = forward_backward(n, ydev, s);
-    if (!e) e = (int)cudaMemcpyAsync(grad, NN.g, sizeof(float) * NN.nparam, cudaMemcpyDeviceToHost, s);
-    if (!e) e = (int)cudaMemcpyAsync(loss, NN.loss_dev, sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (!e) e = (int)cudaMemcpyAsync(NN.y, y, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, s);
+    if (!e) e = forward_backward(n, NN.y, s);
+    if (!e) e = (int)cudaMemcpyAsync(NN.pin ? NN.pin : grad, NN.g, gb, cudaMemcpyDeviceToHost, s);
+    if (!e) e = (int)cudaMemcpyAsync(NN.pin ? (void *)(NN.pin + lo) : loss, NN.loss_dev, sizeof(double),
+                                     cudaMemcpyDeviceToHost, s);
     if (!e) e = (int)cudaStreamSynchronize(s);
-    fk_dfree(ydev);
+    if (!e && NN.pin) {
+        memcpy(grad, NN.pin, gb);
+        memcpy(loss, NN.pin + lo, sizeof(double));
+    }
     *ierr = tc_check(e, "fteik_b200_mlp_gradient");
 }
 
