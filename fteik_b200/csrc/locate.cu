@@ -21,6 +21,15 @@
  * sides, exceeds the event's best objective so far, so the optimum, its
  * index and its ties are those of the full search.  The first best value
  * comes from a strided sample of the points.
+ *
+ * Many events on a fine grid are bounded for 32 points at once first
+ * (l2_block_kernel): over all picks the right-hand side is the square of a
+ * seminorm of the weighted residuals that is zero for a common shift, so with
+ * a block's point c, any tau(g) and d_i = max_g |T_i(g) - T_i(c) - tau(g)|
+ *   sqrt(2 obj(g)) >= sqrt(s2 - s3^2 / sum w^2 at c) - sqrt(sum (w d)^2),
+ * and a block is left out of an event's search if this exceeds the root of
+ * twice its best objective.  tau is the mean over the tables of the
+ * differences, which takes most of the times' common change out of d.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -204,6 +213,318 @@ l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
     }
 }
 
+/* kSlackD: d = max |T(g) - T(c) - tau| of the rounded differences falls short
+ * of the exact one by 2 e d + 2 e |T(g) - T(c)| at most. */
+constexpr float kSlackD = 1.0f / 2097152;  /* 2^-21 = 8 e */
+constexpr int kBlkWarps = 8, kBlkThreads = 32 * kBlkWarps;
+constexpr int kCtaBlk = 32;       /* blocks of 32 points of a CTA */
+constexpr int kCtaPitch = kCtaBlk + 4;
+constexpr int kGroup = 256;       /* events between two loads of the points' tables, at most */
+constexpr int kChunk = 64;        /* events the blocks are tested for at a time */
+constexpr int kBatch = 4;         /* events a warp evaluates at a time */
+constexpr int kParts = 4;         /* the bound's subsets: 16 tables each, l, l + n, l + 2 n, ... of n parts */
+
+/* Tables padded to whole steps of the unrolled loops, and the shared memory
+ * for them: the blocks' centres and departures, and the chunk's picks or the
+ * warps' points and events. */
+__host__ __device__ inline int block_pad(int ntf) { return (ntf + 15) / 16 * 16; }
+__host__ __device__ inline size_t block_smem(int ntf)
+{
+    const size_t per = 2 * kCtaPitch * sizeof(float),
+                 chunk = (kChunk + 2) * sizeof(float2), points = kBlkWarps * (32 * sizeof(float) + kBatch * sizeof(float2));
+    return block_pad(ntf) * (per + (chunk > points ? chunk : points));
+}
+
+/* An event's best objective so far; none yet: a NaN, which rules nothing out. */
+__device__ __forceinline__ float best_so_far(const unsigned long long *best)
+{
+    return __uint_as_float(__ldcg(reinterpret_cast<const unsigned *>(best) + 1));
+}
+
+/* The search of many events by blocks of points (see the file comment).  A CTA
+ * owns 32 blocks.  First each block's T(c) and d go to shared memory.  Then,
+ * for 64 events at a time, a thread bounds 4 blocks x 2 events (3 loads for
+ * 20 packed multiply-adds a pick, bound by those).  Last the points of the
+ * blocks left: a warp takes a block, brings its tables to shared memory and
+ * evaluates four of its events at a time by the point bound, in parts, and
+ * the objective where that does not rule them out.  All loops are short: a
+ * version with the tables in registers and the loops over the picks unrolled
+ * waited for instructions a third of its time (2.7 ms).  New best values go
+ * to all CTAs at once.
+ * 512 events x 64 tables x 2.46e6 points: 6.5 -> 2.1 ms a call, of which the
+ * block bound takes 0.35, its preparation and the picks 0.4, the points 0.9
+ * and the sample 0.2; 64 % of the issue slots are used.  CTAS to an SM: three
+ * up to 48 tables (300 events x 30 x 1.1e6 points: 868 us against 940 with
+ * two), above that the tables' shared memory leaves room for two. */
+template <int CTAS>
+__global__ void __launch_bounds__(kBlkThreads, CTAS)
+l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, int nev, int group,
+                const float *__restrict__ obs, const float *__restrict__ wts, const float *__restrict__ xnorm,
+                unsigned long long *best)
+{
+    extern __shared__ __align__(16) unsigned char block_mem[];
+    __shared__ float2 s_sum[kParts][kChunk];
+    __shared__ float s_is2[kGroup][kParts], s_o2[kGroup], s_xn[kGroup];
+    __shared__ unsigned s_live[kGroup / 32][kCtaBlk];    /* events a block is not ruled out for */
+    __shared__ int s_next;
+    static_assert(kBlkThreads == kParts * kChunk && kChunk == 8 * kBlkWarps && kCtaBlk == 32, "lanes are mapped to these");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = block_pad(ntf), nl = nt / 16;
+    float *const s_c = reinterpret_cast<float *>(block_mem), *const s_d = s_c + nt * kCtaPitch;   /* T at the centres, d */
+    float2 *const s_pk = reinterpret_cast<float2 *>(s_d + nt * kCtaPitch);   /* [nt][kChunk + 2]: w, w o */
+    float4 *const s_ev = reinterpret_cast<float4 *>(s_pk) + warp * (2 * nt);   /* [nt][2]: w, w o of four events */
+    float *const s_t = reinterpret_cast<float *>(reinterpret_cast<float4 *>(s_pk) + kBlkWarps * 2 * nt) + warp * (32 * nt);
+    const long long base = (long long)blockIdx.x * (kCtaBlk * 32);
+    /* a block's tables into the warp's [nt][32]; a lane outside repeats the first point */
+    auto points = [&](long long g0) {
+        const float *src = tables + g0 + (g0 + lane < ngrd ? lane : 0);
+        unsigned dst = (unsigned)__cvta_generic_to_shared(s_t + lane);
+#pragma unroll 8
+        for (int i = 0; i < ntf; ++i, src += ldgrd, dst += 32 * sizeof(float))
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto arrived = [] {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+    };
+    for (int i = ntf; i < nt; ++i) s_t[32 * i + lane] = 0.0f;
+    for (int b = warp; b < kCtaBlk; b += kBlkWarps) { /* the blocks' centres and largest departures */
+        const long long g0 = base + b * 32;
+        if (g0 >= ngrd) break;
+        const int cl = g0 + 16 < ngrd ? 16 : 0;
+        __syncwarp();
+        points(g0);
+        arrived();
+        float sum = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < ntf; ++i) sum += s_t[32 * i + lane];
+        const float tau = (sum - __shfl_sync(0xffffffffu, sum, cl)) / (float)ntf;
+#pragma unroll 8
+        for (int i = 0; i < nt; ++i) {
+            const float c = s_t[32 * i + cl], a = s_t[32 * i + lane] - c;
+            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaf(kSlackD, fabsf(a), fabsf(a - tau))));
+            if (lane == 0) {                              /* a NaN is the largest */
+                s_c[i * kCtaPitch + b] = c;
+                s_d[i * kCtaPitch + b] = __uint_as_float(m);
+            }
+        }
+    }
+    for (long long eg = (long long)blockIdx.y * group; eg < nev; eg += (long long)gridDim.y * group) {
+        const int e0 = (int)eg, n = min(group, nev - e0);
+        __syncthreads();
+        if (tid == 0) s_next = 0;
+        for (int e = tid; e < n; e += kBlkThreads) s_xn[e] = xnorm[e0 + e];
+        s_live[warp][lane] = 0;
+        for (int c0 = 0; c0 < n; c0 += kChunk) {
+            const int nb = min(kChunk, n - c0);
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < kMaxTf; h += 32) {
+                const int i = h + lane;
+                if (h >= nt) break;
+                float o[8], w[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int e = warp + kBlkWarps * k;
+                    const bool on = e < nb && i < ntf;
+                    o[k] = on ? obs[(size_t)(e0 + c0 + e) * ntf + i] : 0.0f;
+                    w[k] = on ? wts[(size_t)(e0 + c0 + e) * ntf + i] : 0.0f;
+                }
+                if (i < nt) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)                  /* a skipped pick has w = 0 */
+                        s_pk[i * (kChunk + 2) + warp + kBlkWarps * k] =
+                            w[k] > 0.0f ? make_float2(w[k], w[k] * o[k]) : make_float2(0.0f, 0.0f);
+                }
+            }
+            __syncthreads();
+            if (tid < kChunk * nl) {   /* 64 threads a part, one an event: sum w^2 and sum (w o)^2 */
+                const int e = tid % kChunk, k = tid / kChunk;
+                float a = 0.0f, o2 = 0.0f;
+#pragma unroll 4
+                for (int i = k; i < nt; i += nl) {
+                    const float2 p = s_pk[i * (kChunk + 2) + e];
+                    a = fmaf(p.x, p.x, a);
+                    o2 = fmaf(p.y, p.y, o2);
+                }
+                s_sum[k][e] = make_float2(a, o2);
+            }
+            __syncthreads();
+            if (tid < kChunk) {
+                float a = 0.0f, o2 = 0.0f;
+                for (int k = 0; k < nl; ++k) {
+                    a += s_sum[k][tid].x;
+                    o2 += s_sum[k][tid].y;
+                    s_is2[c0 + tid][k] = a > 0.0f ? 1.0f / a : 0.0f;
+                }
+                s_o2[c0 + tid] = kSlackO2 * o2;
+            }
+            __syncthreads();
+            /* the blocks: 4 of them (two packed pairs) and 2 events to a thread */
+            const int b0 = 4 * (lane & 7), ev = 8 * warp + 2 * (lane >> 3);
+            float2 s2[2][2], s3[2][2], d2[2][2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s2[k / 2][k % 2] = s3[k / 2][k % 2] = d2[k / 2][k % 2] = dup(0.0f);
+#pragma unroll 4
+            for (int i = 0; i < nt; ++i) {
+                const float4 c = *reinterpret_cast<const float4 *>(s_c + i * kCtaPitch + b0);
+                const float4 d = *reinterpret_cast<const float4 *>(s_d + i * kCtaPitch + b0);
+                const float4 pk = *reinterpret_cast<const float4 *>(s_pk + i * (kChunk + 2) + ev);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float2 w = dup(k ? pk.z : pk.x), nw = dup(k ? -pk.z : -pk.x), wo = dup(k ? pk.w : pk.y);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float2 p = __ffma2_rn(nw, j ? make_float2(c.z, c.w) : make_float2(c.x, c.y), wo);
+                        const float2 r = __fmul2_rn(w, j ? make_float2(d.z, d.w) : make_float2(d.x, d.y));
+                        s2[k][j] = __ffma2_rn(p, p, s2[k][j]);
+                        s3[k][j] = __ffma2_rn(w, p, s3[k][j]);
+                        d2[k][j] = __ffma2_rn(r, r, d2[k][j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int e = c0 + ev + k;
+                if (ev + k >= nb) break;
+                const float is2 = s_is2[e][nl - 1], o2 = s_o2[e], u = best_so_far(best + e0 + e);
+                const float root = sqrtf(fmaf(2.0f * u, 1.0f + kSlackObj, o2));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float a = j & 1 ? s2[k][j / 2].y : s2[k][j / 2].x, b = j & 1 ? s3[k][j / 2].y : s3[k][j / 2].x;
+                    const float dd = j & 1 ? d2[k][j / 2].y : d2[k][j / 2].x;
+                    const float lb = fmaf(-b * is2, b, fmaf(a, -kSlackS2, a)) - o2;
+                    const float need = (root + fmaf(sqrtf(dd), 1.0f + kSlackS2, 1e-18f)) * (1.0f + kSlackO2);
+                    if (base + (b0 + j) * 32 < ngrd && !(sqrtf(fmaxf(lb, 0.0f)) > need))
+                        atomicOr(&s_live[e / 32][b0 + j], 1u << (e & 31));
+                }
+            }
+        }
+        __syncthreads();
+        for (int i = ntf; i < nt; ++i) s_t[32 * i + lane] = 0.0f;
+        /* the points of the blocks left: a block to a warp, four events at a time */
+        for (;;) {
+            int b = 0;
+            if (lane == 0) b = atomicAdd(&s_next, 1);
+            b = __shfl_sync(0xffffffffu, b, 0);
+            if (b >= kCtaBlk) break;
+            const unsigned mine = lane < kGroup / 32 ? s_live[lane][b] : 0;
+            if (!__any_sync(0xffffffffu, mine)) continue;
+            __syncwarp();
+            points(base + b * 32);
+            const long long gl = base + b * 32 + lane;
+            const bool in = gl < ngrd;
+            const int g = in ? (int)gl : 0;
+            int q = -1, ne[kBatch];                          /* the next events and their picks */
+            unsigned left = 0;
+            float po[kBatch][kMaxTf / 32] = {}, pw[kBatch][kMaxTf / 32] = {}, pu[kBatch];
+            auto fetch = [&]() {
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    while (!left && q < kGroup / 32) left = __shfl_sync(0xffffffffu, mine, ++q);
+                    ne[k] = left ? 32 * q + __ffs(left) - 1 : -1;
+                    left &= left - 1;
+                    pu[k] = ne[k] >= 0 ? best_so_far(best + e0 + ne[k]) : 0.0f;
+#pragma unroll
+                    for (int h = 0; h < kMaxTf / 32; ++h) {
+                        if (h > 0 && 32 * h >= ntf) break;
+                        const bool on = ne[k] >= 0 && 32 * h + lane < ntf;
+                        po[k][h] = on ? __ldg(obs + (size_t)(e0 + ne[k]) * ntf + 32 * h + lane) : 0.0f;
+                        pw[k][h] = on ? __ldg(wts + (size_t)(e0 + ne[k]) * ntf + 32 * h + lane) : 0.0f;
+                    }
+                }
+            };
+            fetch();
+            arrived();
+            while (ne[0] >= 0) {
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < kMaxTf / 32; ++h) {
+                    if (h > 0 && 32 * h >= nt) break;
+                    float4 v[2];
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const float w = pw[k][h] > 0.0f ? pw[k][h] : 0.0f, wo = pw[k][h] > 0.0f ? w * po[k][h] : 0.0f;
+                        if (k & 1) { v[k / 2].z = w; v[k / 2].w = wo; } else { v[k / 2].x = w; v[k / 2].y = wo; }
+                    }
+                    if (32 * h + lane < nt) {
+                        s_ev[2 * (32 * h + lane)] = v[0];
+                        s_ev[2 * (32 * h + lane) + 1] = v[1];
+                    }
+                }
+                __syncwarp();
+                int e[kBatch];
+                bool x[kBatch];
+                float thr[kBatch], s2[kBatch], s3[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    x[k] = ne[k] >= 0;
+                    e[k] = x[k] ? ne[k] : ne[0];
+                    thr[k] = fmaf(2.0f * pu[k], 1.0f + kSlackObj, s_o2[e[k]]);
+                    s2[k] = s3[k] = 0.0f;
+                }
+                fetch();
+#pragma unroll 1
+                for (int l = 0; l < nl; ++l) {
+                    const float *pt = s_t + 32 * l + lane;
+                    const float4 *pe = s_ev + 2 * l;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, pt += 32 * nl, pe += 2 * nl) {
+                        const float t = *pt;
+                        const float4 pa = pe[0], pb = pe[1];
+                        const float w[kBatch] = {pa.x, pa.z, pb.x, pb.z}, wo[kBatch] = {pa.y, pa.w, pb.y, pb.w};
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k) {
+                            const float p = fmaf(-w[k], t, wo[k]);
+                            s2[k] = fmaf(p, p, s2[k]);
+                            s3[k] = fmaf(w[k], p, s3[k]);
+                        }
+                    }
+                    bool any = false;
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const float lb = fmaf(-s3[k] * s_is2[e[k]][l], s3[k], fmaf(s2[k], -kSlackS2, s2[k]));
+                        x[k] = __any_sync(0xffffffffu, in && x[k] && !(lb > thr[k]));
+                        any |= x[k];
+                    }
+                    if (!any) break;
+                }
+#pragma unroll 1
+                for (int k = 0; k < kBatch; ++k) {
+                    const bool on = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
+                    if (!on) continue;
+                    const int ek = k == 0 ? e[0] : k == 1 ? e[1] : k == 2 ? e[2] : e[3];
+                    float o[kMaxTf / 32], w[kMaxTf / 32];
+#pragma unroll
+                    for (int h = 0; h < kMaxTf / 32; ++h) {
+                        const bool use = 32 * h + lane < ntf;
+                        o[h] = use ? __ldg(obs + (size_t)(e0 + ek) * ntf + 32 * h + lane) : 0.0f;
+                        w[h] = use ? __ldg(wts + (size_t)(e0 + ek) * ntf + 32 * h + lane) : 0.0f;
+                    }
+                    const float xn = s_xn[ek];
+                    float t0 = 0.0f, obj = 0.0f;             /* as l2_search_kernel's, in its order */
+#pragma unroll 4
+                    for (int i = 0; i < ntf; ++i) {
+                        const float oi = __shfl_sync(0xffffffffu, i < 32 ? o[0] : o[1], i & 31);
+                        const float wi = __shfl_sync(0xffffffffu, i < 32 ? w[0] : w[1], i & 31);
+                        const float t = __fadd_rn(t0, __fmul_rn(wi, __fmul_rn(xn, __fsub_rn(oi, s_t[32 * i + lane]))));
+                        t0 = wi > 0.0f ? t : t0;
+                    }
+#pragma unroll 4
+                    for (int i = 0; i < ntf; ++i) {
+                        const float oi = __shfl_sync(0xffffffffu, i < 32 ? o[0] : o[1], i & 31);
+                        const float wi = __shfl_sync(0xffffffffu, i < 32 ? w[0] : w[1], i & 31);
+                        const float res = __fmul_rn(__fmul_rn(0.70710677f, wi), __fsub_rn(oi, __fadd_rn(s_t[32 * i + lane], t0)));
+                        obj = wi > 0.0f ? __fadd_rn(obj, __fmul_rn(res, res)) : obj;
+                    }
+                    const unsigned long long key = warp_min(in ? pack_key(obj, g) : ~0ull);
+                    if (lane == 0) atomicMin(best + e0 + ek, key);
+                }
+            }
+        }
+    }
+}
+
 /* t0 and obj at the optimum, same arithmetic: a warp per event fetches its
  * 64 terms at once, one lane adds them in order. */
 __global__ void __launch_bounds__(128)
@@ -260,6 +581,16 @@ __global__ void xnorm_kernel(int nev, int ntf, const float *__restrict__ wts, fl
  * x 20 tables x 168,000 points: 118 us against 303. */
 constexpr int kBoundEvents = 8, kBoundPoints = 4096;
 constexpr int kSample = 256;
+/* Blocks of points pay from about 200 events (their centres and departures
+ * cost as much as some 100 events' point bounds) and on fine grids, where the
+ * times change little within 32 points; above 48 tables two CTAs share an SM
+ * instead of three and the grid has to be larger.  By points / by blocks, us:
+ * 192 events x 269e3 points x 14, 30, 60 tables 198 / 183, 249 / 243, 387 / 412;
+ * x 542e3 x 60 673 / 668; x 1.09e6 x 60 1311 / 1141; 60 events x 600e3 x 20
+ * 183 / 207; 300 events x 99e3 x 32 210 / 250; 500 events x 256e3 x 20
+ * 496 / 382. */
+constexpr int kBlockEvents = 192;
+inline int block_points(int ntf) { return ntf <= 48 ? 1 << 18 : 1 << 19; }
 
 /* CTAs over the events when the points alone leave the chip idle (148 SMs,
  * 3 CTAs each, a few waves) */
@@ -271,7 +602,7 @@ inline int event_split(long long ctas, int nev)
 }
 
 template <int NTF>
-void launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
+cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
                       const float *xn, unsigned long long *best, cudaStream_t s)
 {
     const int per = kThreads / 32 * 64;
@@ -279,12 +610,28 @@ void launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev
     const dim3 grid((unsigned)ctas, event_split(ctas, nev));
     if (nev < kBoundEvents || ngrd < kBoundPoints) {
         l2_search_kernel<NTF, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, xn, best);
-        return;
+        return cudaSuccess;
     }
     const long long cs = ((ngrd + kSample - 1) / kSample + (long long)per - 1) / per;
     l2_search_kernel<NTF, false><<<dim3((unsigned)cs, event_split(cs, nev)), kThreads, 0, s>>>(
         ngrd, ldgrd, ntf, kSample, tables, nev, obs, wts, xn, best);
-    l2_search_kernel<NTF, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, xn, best);
+    if (nev < kBlockEvents || ngrd < block_points(ntf)) {
+        l2_search_kernel<NTF, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, xn, best);
+        return cudaSuccess;
+    }
+    const long long cb = (ngrd + 32ll * kCtaBlk - 1) / (32 * kCtaBlk);
+    /* events in groups, smaller ones when the points alone leave the chip idle */
+    int group = kGroup;
+    while (group > kChunk && cb * ((nev + group - 1) / group) < 148 * 2 * 4) group /= 2;
+    long long y = (148 * 2 * 4 + cb - 1) / cb;
+    const long long ng = (nev + group - 1) / group;
+    const size_t smem = block_smem(ntf);
+    auto *kernel = ntf <= 48 ? l2_block_kernel<3> : l2_block_kernel<2>;
+    const cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ea != cudaSuccess) return ea;
+    kernel<<<dim3((unsigned)cb, (unsigned)(y < 1 ? 1 : y > ng ? ng : y)), kBlkThreads, smem, s>>>(
+        ngrd, ldgrd, ntf, tables, nev, group, obs, wts, xn, best);
+    return cudaSuccess;
 }
 
 } // namespace
@@ -306,9 +653,9 @@ extern "C" int fk_locate_l2_exact(int ngrd, int ldgrd, int ntf, const float *tab
     unsigned long long *best = (unsigned long long *)scratch;
     float *xn = (float *)(best + nev);
     xnorm_kernel<<<(nev + 127) / 128, 128, 0, s>>>(nev, ntf, wts, xn, best);
-    if (ntf <= 16) launch_l2_search<16>(ngrd, ldgrd, ntf, tables, nev, obs, wts, xn, best, s);
-    else if (ntf <= 32) launch_l2_search<32>(ngrd, ldgrd, ntf, tables, nev, obs, wts, xn, best, s);
-    else launch_l2_search<64>(ngrd, ldgrd, ntf, tables, nev, obs, wts, xn, best, s);
+    auto *search = ntf <= 16 ? launch_l2_search<16> : ntf <= 32 ? launch_l2_search<32> : launch_l2_search<64>;
+    const cudaError_t e = search(ngrd, ldgrd, ntf, tables, nev, obs, wts, xn, best, s);
+    if (e != cudaSuccess) return (int)e;
     l2_at_opt_kernel<<<(nev + 3) / 4, 128, 0, s>>>(ldgrd, ntf, tables, nev, obs, wts, xn, best, out_idx, out_t0,
                                                    out_obj);
     return (int)cudaGetLastError();
