@@ -78,7 +78,7 @@ constexpr float kSlackO2 = 1.0f / 1048576; /* 2^-20 = 16 e */
  * costs 3 packed operations and one 16-byte shared-memory broadcast a pick. */
 template <int NTF, bool BOUND>
 __global__ void __launch_bounds__(kThreads, NTF == 64 ? 3 : 4)
-l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restrict__ tables, int nev,
+l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restrict__ tables, int nev, int chunk,
                  const float *__restrict__ obs, const float *__restrict__ wts,
                  const float *__restrict__ xnorm, unsigned long long *best)
 {
@@ -100,9 +100,9 @@ l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
         if (i < ntf && in1) b = __ldg(tables + (size_t)i * ldgrd + g1);
         nT[i] = make_float2(-a, -b);
     }
-    const int nchunk = (nev + kEvChunk - 1) / kEvChunk;
+    const int nchunk = (nev + chunk - 1) / chunk;
     for (int c = blockIdx.y; c < nchunk; c += gridDim.y) {
-        const int e0 = c * kEvChunk, nb = min(kEvChunk, nev - e0);
+        const int e0 = c * chunk, nb = min(chunk, nev - e0);
         __syncthreads();
 #pragma unroll 1
         for (int t = threadIdx.x; t < kEvChunk * NTF; t += kThreads) {
@@ -241,6 +241,23 @@ __device__ __forceinline__ float best_so_far(const unsigned long long *best)
     return __uint_as_float(__ldcg(reinterpret_cast<const unsigned *>(best) + 1));
 }
 
+/* A block's tables into a warp's t[ntf][32]; a lane outside repeats the first point. */
+__device__ __forceinline__ void block_points(float *t, const float *__restrict__ tables, int ldgrd, int ntf, int ngrd,
+                                             long long g0, int lane)
+{
+    const float *src = tables + g0 + (g0 + lane < ngrd ? lane : 0);
+    unsigned dst = (unsigned)__cvta_generic_to_shared(t + lane);
+#pragma unroll 8
+    for (int i = 0; i < ntf; ++i, src += ldgrd, dst += 32 * sizeof(float))
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void block_arrived()
+{
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+}
+
 /* The search of many events by blocks of points (see the file comment).  A CTA
  * owns 32 blocks.  First each block's T(c) and d go to shared memory.  Then,
  * for 64 events at a time, a thread bounds 4 blocks x 2 events (3 loads for
@@ -274,27 +291,14 @@ l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
     float4 *const s_ev = reinterpret_cast<float4 *>(s_pk) + warp * (2 * nt);   /* [nt][2]: w, w o of four events */
     float *const s_t = reinterpret_cast<float *>(reinterpret_cast<float4 *>(s_pk) + kBlkWarps * 2 * nt) + warp * (32 * nt);
     const long long base = (long long)blockIdx.x * (kCtaBlk * 32);
-    /* a block's tables into the warp's [nt][32]; a lane outside repeats the first point */
-    auto points = [&](long long g0) {
-        const float *src = tables + g0 + (g0 + lane < ngrd ? lane : 0);
-        unsigned dst = (unsigned)__cvta_generic_to_shared(s_t + lane);
-#pragma unroll 8
-        for (int i = 0; i < ntf; ++i, src += ldgrd, dst += 32 * sizeof(float))
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto arrived = [] {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();
-    };
     for (int i = ntf; i < nt; ++i) s_t[32 * i + lane] = 0.0f;
     for (int b = warp; b < kCtaBlk; b += kBlkWarps) { /* the blocks' centres and largest departures */
         const long long g0 = base + b * 32;
         if (g0 >= ngrd) break;
         const int cl = g0 + 16 < ngrd ? 16 : 0;
         __syncwarp();
-        points(g0);
-        arrived();
+        block_points(s_t, tables, ldgrd, ntf, ngrd, g0, lane);
+        block_arrived();
         float sum = 0.0f;
 #pragma unroll 8
         for (int i = 0; i < ntf; ++i) sum += s_t[32 * i + lane];
@@ -411,7 +415,7 @@ l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
             const unsigned mine = lane < kGroup / 32 ? s_live[lane][b] : 0;
             if (!__any_sync(0xffffffffu, mine)) continue;
             __syncwarp();
-            points(base + b * 32);
+            block_points(s_t, tables, ldgrd, ntf, ngrd, base + b * 32, lane);
             const long long gl = base + b * 32 + lane;
             const bool in = gl < ngrd;
             const int g = in ? (int)gl : 0;
@@ -435,7 +439,7 @@ l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
                 }
             };
             fetch();
-            arrived();
+            block_arrived();
             while (ne[0] >= 0) {
                 __syncwarp();
 #pragma unroll
@@ -592,13 +596,27 @@ constexpr int kSample = 256;
 constexpr int kBlockEvents = 192;
 inline int block_points(int ntf) { return ntf <= 48 ? 1 << 18 : 1 << 19; }
 
-/* CTAs over the events when the points alone leave the chip idle (148 SMs,
- * 3 CTAs each, a few waves) */
-inline int event_split(long long ctas, int nev)
+/* Grid of the point kernels: their CTAs over the points, and over the events
+ * when those leave the chip idle (148 SMs, 3 CTAs each, a few waves); chunks of
+ * fewer events when that still does, as in the sample of a small grid. */
+inline dim3 point_grid(long long ctas, int nev, int *chunk)
 {
-    const int nchunk = (nev + kEvChunk - 1) / kEvChunk;
-    long long y = (148 * 3 * 4 + ctas - 1) / ctas;
-    return (int)(y < 1 ? 1 : y > nchunk ? nchunk : y);
+    *chunk = kEvChunk;
+    while (*chunk > 1 && ctas * ((nev + *chunk - 1) / *chunk) < 148 * 3) *chunk /= 2;
+    const int nchunk = (nev + *chunk - 1) / *chunk;
+    const long long y = (148 * 3 * 4 + ctas - 1) / ctas;
+    return dim3((unsigned)ctas, (unsigned)(y < 1 ? 1 : y > nchunk ? nchunk : y));
+}
+
+/* Grid of the block kernels: the blocks, and events in groups, smaller ones
+ * when the points alone leave the chip idle. */
+inline dim3 block_grid(int ngrd, int nev, int *group)
+{
+    const long long cb = (ngrd + 32ll * kCtaBlk - 1) / (32 * kCtaBlk);
+    *group = kGroup;
+    while (*group > kChunk / 2 && cb * ((nev + *group - 1) / *group) < 148 * 2 * 4) *group /= 2;
+    const long long y = (148 * 2 * 4 + cb - 1) / cb, ng = (nev + *group - 1) / *group;
+    return dim3((unsigned)cb, (unsigned)(y < 1 ? 1 : y > ng ? ng : y));
 }
 
 template <int NTF>
@@ -607,29 +625,28 @@ cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, 
 {
     const int per = kThreads / 32 * 64;
     const long long ctas = (ngrd + (long long)per - 1) / per;
-    const dim3 grid((unsigned)ctas, event_split(ctas, nev));
+    int chunk;
+    const dim3 grid = point_grid(ctas, nev, &chunk);
     if (nev < kBoundEvents || ngrd < kBoundPoints) {
-        l2_search_kernel<NTF, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, xn, best);
+        l2_search_kernel<NTF, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, xn, best);
         return cudaSuccess;
     }
     const long long cs = ((ngrd + kSample - 1) / kSample + (long long)per - 1) / per;
-    l2_search_kernel<NTF, false><<<dim3((unsigned)cs, event_split(cs, nev)), kThreads, 0, s>>>(
-        ngrd, ldgrd, ntf, kSample, tables, nev, obs, wts, xn, best);
+    int schunk;
+    const dim3 sgrid = point_grid(cs, nev, &schunk);
+    l2_search_kernel<NTF, false><<<sgrid, kThreads, 0, s>>>(
+        ngrd, ldgrd, ntf, kSample, tables, nev, schunk, obs, wts, xn, best);
     if (nev < kBlockEvents || ngrd < block_points(ntf)) {
-        l2_search_kernel<NTF, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, xn, best);
+        l2_search_kernel<NTF, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, xn, best);
         return cudaSuccess;
     }
-    const long long cb = (ngrd + 32ll * kCtaBlk - 1) / (32 * kCtaBlk);
-    /* events in groups, smaller ones when the points alone leave the chip idle */
-    int group = kGroup;
-    while (group > kChunk && cb * ((nev + group - 1) / group) < 148 * 2 * 4) group /= 2;
-    long long y = (148 * 2 * 4 + cb - 1) / cb;
-    const long long ng = (nev + group - 1) / group;
+    int group;
+    const dim3 gb = block_grid(ngrd, nev, &group);
     const size_t smem = block_smem(ntf);
     auto *kernel = ntf <= 48 ? l2_block_kernel<3> : l2_block_kernel<2>;
     const cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ea != cudaSuccess) return ea;
-    kernel<<<dim3((unsigned)cb, (unsigned)(y < 1 ? 1 : y > ng ? ng : y)), kBlkThreads, smem, s>>>(
+    kernel<<<gb, kBlkThreads, smem, s>>>(
         ngrd, ldgrd, ntf, tables, nev, group, obs, wts, xn, best);
     return cudaSuccess;
 }
@@ -731,7 +748,8 @@ extern "C" void fteik_b200_locate_l2_noalloc(int ngrd, int ldgrd, int ntf, const
 /* A thread holds the 64 residuals of one grid point in registers and sorts */
 /* them with a fully unrolled bitonic network (skipped picks sort last as   */
 /* +inf); the half sums use compile-time indices.  Most points are ruled    */
-/* out first by a bound on the misfit (l1_search_kernel).  The argmin is    */
+/* out first by a bound on the misfit (l1_search_kernel), of many events on */
+/* large grids 32 at a time (l1_block_kernel).  The argmin is               */
 /* the first-index minimum (64-bit atomicMin on (bits << 32) | g); t0 and   */
 /* obj at the optimum are recomputed in FP64.                               */
 /* ------------------------------------------------------------------------ */
@@ -757,6 +775,23 @@ __device__ __forceinline__ void bitonic_sort(float (&v)[N])
             }
 }
 
+/* Misfit per unit weight of n residuals (the others +inf); sorts them. */
+template <int N>
+__device__ __forceinline__ float l1_sorted_misfit(float (&r)[N], int n)
+{
+    bitonic_sort<N>(r);
+    const int h = n / 2;
+    float obj = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        /* lower half: i < h; upper half: n - h <= i < n (the middle one of
+         * an odd count drops out) */
+        const float cf = i < h ? -1.0f : ((i >= n - h && i < n) ? 1.0f : 0.0f);
+        obj = fmaf(cf, (i < n) ? r[i] : 0.0f, obj);
+    }
+    return obj;
+}
+
 /* Rounding allowance of the L1 bound: with e = 2^-24 the ranking misfit is
  * computed to (N + 1) e sum (|o| + |T|) and the pairs' sum to (N / 2 + 4) e of
  * the same, N <= 64 (times the event's weight). */
@@ -765,7 +800,7 @@ constexpr float kSlackL1 = 1.0f / 131072;   /* 2^-17 = 128 e */
 /* Searches the points p stride; a warp owns 32 points, one a lane, and runs
  * over the events as l2_search_kernel does.  BOUND: for any t0 two picks
  * give |r_i - t0| + |r_j - t0| >= |r_i - r_j|, so the sum over disjoint pairs
- * (i, i + N / 2) bounds the misfit from below at four operations a pair,
+ * (2 i, 2 i + 1) bounds the misfit from below at four operations a pair,
  * against the sorting network's 672 compare-exchanges for 64 picks; the
  * pairs come in kLevels levels, and a point is sorted only if all of them
  * stay below the event's best misfit so far.  A pair with a skipped pick
@@ -774,7 +809,7 @@ constexpr float kSlackL1 = 1.0f / 131072;   /* 2^-17 = 128 e */
  * 38.6 ms with every point sorted. */
 template <int N, bool BOUND>
 __global__ void __launch_bounds__(kThreads, 3)
-l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restrict__ tables, int nev,
+l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restrict__ tables, int nev, int chunk,
                  const float *__restrict__ obs, const float *__restrict__ wts, unsigned long long *best)
 {
     __shared__ float s_obs[kEvChunk][N];
@@ -795,9 +830,9 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
         T[i] = (in && i < ntf) ? __ldg(tables + (size_t)i * ldgrd + g) : 0.0f;
         sumT += fabsf(T[i]);
     }
-    const int nchunk = (nev + kEvChunk - 1) / kEvChunk;
+    const int nchunk = (nev + chunk - 1) / chunk;
     for (int c = blockIdx.y; c < nchunk; c += gridDim.y) {
-        const int e0 = c * kEvChunk, nb = min(kEvChunk, nev - e0);
+        const int e0 = c * chunk, nb = min(chunk, nev - e0);
         __syncthreads();
 #pragma unroll 1
         for (int t = threadIdx.x; t < kEvChunk * N; t += kThreads) {
@@ -815,8 +850,8 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
                 if (s_w[e][i] > 0.0f) { ++n; wv = s_w[e][i]; so += fabsf(s_obs[e][i]); }
             if (BOUND)
                 for (int i = lane; i < N / 2; i += 32)
-                    s_pair[e][i] = make_float2(s_obs[e][i] - s_obs[e][i + N / 2],
-                                               s_w[e][i] > 0.0f && s_w[e][i + N / 2] > 0.0f ? INF : 0.0f);
+                    s_pair[e][i] = make_float2(s_obs[e][2 * i] - s_obs[e][2 * i + 1],
+                                               s_w[e][2 * i] > 0.0f && s_w[e][2 * i + 1] > 0.0f ? INF : 0.0f);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 n += __shfl_xor_sync(0xffffffffu, n, o);
@@ -847,7 +882,7 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
 #pragma unroll
                     for (int i = l; i < N / 2; i += kLevels) {
                         const float2 q = s_pair[e][i];
-                        la += fminf(fabsf(q.x - (T[i] - T[i + N / 2])), q.y);
+                        la += fminf(fabsf(q.x - (T[2 * i] - T[2 * i + 1])), q.y);
                     }
                     any = __any_sync(0xffffffffu, in && !(la > thr));
                     if (!any) break;
@@ -857,17 +892,8 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
             float r[N];
 #pragma unroll
             for (int i = 0; i < N; ++i) r[i] = s_w[e][i] > 0.0f ? s_obs[e][i] - T[i] : INF;
-            bitonic_sort<N>(r);
-            const int n = s_n[e], h = n / 2;
-            float obj = 0.0f;
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-                /* lower half: i < h; upper half: n - h <= i < n (the middle one of
-                 * an odd count drops out) */
-                const float cf = i < h ? -1.0f : ((i >= n - h && i < n) ? 1.0f : 0.0f);
-                obj = fmaf(cf, (i < n) ? r[i] : 0.0f, obj);
-            }
-            obj *= s_wv[e];
+            const int n = s_n[e];
+            const float obj = l1_sorted_misfit<N>(r, n) * s_wv[e];
             const unsigned long long key = warp_min((in && n > 0) ? pack_key(obj, g) : ~0ull);
             if (lane == 0) {
                 atomicMin(&s_best[e], key);
@@ -879,21 +905,267 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
     }
 }
 
-/* One or two launches, as launch_l2_search. */
+/* Shared memory of l1_block_kernel: a block's pairs at its centre and their
+ * departures, and the chunk's pairs or the warps' points, events and picks. */
+__host__ __device__ inline int l1_pairs_pad(int ntf) { return (ntf / 2 + 7) / 8 * 8; }
+inline size_t l1_block_smem(int ntf)
+{
+    const size_t np = l1_pairs_pad(ntf), per = 2 * kCtaPitch * np, chunk = (kChunk + 2) * np,
+                 points = kBlkWarps * (32 * ntf + kBatch * np + 2 * kMaxTf);
+    return sizeof(float) * (per + (chunk > points ? chunk : points));
+}
+
+/* The search of many events by blocks of 32 points, as l2_block_kernel.  The
+ * bound's pairs are picks i and i + ntf / 2: with a block's centre c and
+ * d = max_g |(T_i - T_j)(g) - (T_i - T_j)(c)| a pair gives at least
+ * max(0, |o_i - o_j - (T_i - T_j)(c)| - d) anywhere in the block.  A pair with
+ * a skipped pick is a NaN, which the maximum turns into zero.  The rounding
+ * errors of the bound, (N / 2 + 6) e of sum |o|, sum |T| and the departures,
+ * and of the ranking misfit stay below twice kSlackL1 (|o| + |T|).
+ * 128 events x 64 tables x 2.46e6 points: 3.3 -> 1.28 ms a call. */
 template <int N>
-void launch_l1_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
+__global__ void __launch_bounds__(kBlkThreads, N == 64 ? 2 : 3)
+l1_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, int nev, int group,
+                const float *__restrict__ obs, const float *__restrict__ wts, unsigned long long *best)
+{
+    extern __shared__ __align__(16) unsigned char block_mem[];
+    __shared__ float s_wv[kGroup], s_o[kGroup], s_far[kCtaBlk];   /* weight, sum |o|; largest sum |T| */
+    __shared__ int s_n[kGroup];
+    __shared__ unsigned s_live[kGroup / 32][kCtaBlk];
+    __shared__ int s_next;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = ntf / 2, np = l1_pairs_pad(ntf);
+    const float INF = __int_as_float(0x7f800000), NONE = __int_as_float(0x7fffffff);
+    float *const s_c = reinterpret_cast<float *>(block_mem), *const s_d = s_c + np * kCtaPitch;
+    float *const s_q = s_d + np * kCtaPitch;                        /* [np][kChunk + 2]: o_i - o_j */
+    float4 *const s_ev = reinterpret_cast<float4 *>(s_q) + warp * np;   /* of four events */
+    float2 *const s_ow = reinterpret_cast<float2 *>(reinterpret_cast<float4 *>(s_q) + kBlkWarps * np) + warp * kMaxTf;
+    float *const s_t = s_q + kBlkWarps * (kBatch * np + 2 * kMaxTf) + warp * (32 * ntf);
+    const long long base = (long long)blockIdx.x * (kCtaBlk * 32);
+    for (int b = warp; b < kCtaBlk; b += kBlkWarps) {
+        const long long g0 = base + b * 32;
+        if (g0 >= ngrd) break;
+        const int cl = g0 + 16 < ngrd ? 16 : 0;
+        __syncwarp();
+        block_points(s_t, tables, ldgrd, ntf, ngrd, g0, lane);
+        block_arrived();
+        float sum = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < ntf; ++i) sum += fabsf(s_t[32 * i + lane]);
+        const unsigned far = __reduce_max_sync(0xffffffffu, __float_as_uint(sum));
+        if (lane == 0) s_far[b] = __uint_as_float(far);
+#pragma unroll 4
+        for (int i = 0; i < np; ++i) {
+            float c = 0.0f;
+            unsigned m = 0;
+            if (i < half) {
+                const float t = s_t[32 * i + lane] - s_t[32 * (i + half) + lane];
+                c = __shfl_sync(0xffffffffu, t, cl);
+                m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(t - c)));   /* a NaN is the largest */
+            }
+            if (lane == 0) {
+                s_c[i * kCtaPitch + b] = c;
+                s_d[i * kCtaPitch + b] = __uint_as_float(m);
+            }
+        }
+    }
+    for (long long eg = (long long)blockIdx.y * group; eg < nev; eg += (long long)gridDim.y * group) {
+        const int e0 = (int)eg, n = min(group, nev - e0);
+        __syncthreads();
+        if (tid == 0) s_next = 0;
+        s_live[warp][lane] = 0;
+        for (int c0 = 0; c0 < n; c0 += kChunk) {
+            const int nb = min(kChunk, n - c0);
+            __syncthreads();
+#pragma unroll 4
+            for (int k = 0; k < kChunk / kBlkWarps; ++k) {       /* a warp an event, a lane a pair */
+                const int e = warp + kBlkWarps * k;
+                const float *po = obs + (size_t)(e0 + c0 + e) * ntf, *pw = wts + (size_t)(e0 + c0 + e) * ntf;
+                const bool a = e < nb && lane < half, last = e < nb && lane == 0 && (ntf & 1);
+                const float oi = a ? po[lane] : 0.0f, wi = a ? pw[lane] : 0.0f;
+                const float oj = a ? po[lane + half] : 0.0f, wj = a ? pw[lane + half] : 0.0f;
+                const float ol = last ? po[ntf - 1] : 0.0f, wl = last ? pw[ntf - 1] : 0.0f;
+                const bool ui = wi > 0.0f, uj = wj > 0.0f, ul = wl > 0.0f;
+                const int cnt = __popc(__ballot_sync(0xffffffffu, ui)) + __popc(__ballot_sync(0xffffffffu, uj)) +
+                                __popc(__ballot_sync(0xffffffffu, ul));
+                const unsigned wv = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(ui ? wi : 0.0f, uj ? wj : 0.0f),
+                                                                                        ul ? wl : 0.0f)));
+                float so = (ui ? fabsf(oi) : 0.0f) + (uj ? fabsf(oj) : 0.0f) + (ul ? fabsf(ol) : 0.0f);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) so += __shfl_xor_sync(0xffffffffu, so, o);
+                if (lane < np) s_q[lane * (kChunk + 2) + e] = ui && uj ? oi - oj : NONE;
+                if (lane == 0) {
+                    s_n[c0 + e] = cnt;
+                    s_wv[c0 + e] = __uint_as_float(wv);       /* one weight per event */
+                    s_o[c0 + e] = so;
+                }
+            }
+            __syncthreads();
+            const int b0 = 4 * (lane & 7), ev = 8 * warp + 2 * (lane >> 3);
+            float la[2][4] = {};
+#pragma unroll 8
+            for (int i = 0; i < np; ++i) {
+                const float4 c4 = *reinterpret_cast<const float4 *>(s_c + i * kCtaPitch + b0);
+                const float4 d4 = *reinterpret_cast<const float4 *>(s_d + i * kCtaPitch + b0);
+                const float2 q = *reinterpret_cast<const float2 *>(s_q + i * (kChunk + 2) + ev);
+                const float c[4] = {c4.x, c4.y, c4.z, c4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    la[0][j] += fmaxf(fabsf(q.x - c[j]) - d[j], 0.0f);
+                    la[1][j] += fmaxf(fabsf(q.y - c[j]) - d[j], 0.0f);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int e = c0 + ev + k;
+                if (ev + k >= nb) break;
+                const float u = best_so_far(best + e0 + e), most = u / s_wv[e] * (1.0f + 1.0f / 1048576);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    /* a misfit of -0 or rounded below zero orders after all others (its key is unsigned) */
+                    const float thr = signbit(u) ? INF : fmaf(2.0f * kSlackL1, s_far[b0 + j] + s_o[e], most);
+                    if (base + (b0 + j) * 32 < ngrd && !(la[k][j] > thr)) atomicOr(&s_live[e / 32][b0 + j], 1u << (e & 31));
+                }
+            }
+        }
+        __syncthreads();
+        for (;;) {
+            int b = 0;
+            if (lane == 0) b = atomicAdd(&s_next, 1);
+            b = __shfl_sync(0xffffffffu, b, 0);
+            if (b >= kCtaBlk) break;
+            const unsigned mine = lane < kGroup / 32 ? s_live[lane][b] : 0;
+            if (!__any_sync(0xffffffffu, mine)) continue;
+            __syncwarp();
+            block_points(s_t, tables, ldgrd, ntf, ngrd, base + b * 32, lane);
+            const long long gl = base + b * 32 + lane;
+            const bool in = gl < ngrd;
+            const int g = in ? (int)gl : 0;
+            int q = -1, ne[kBatch];                              /* the next events and their pairs */
+            unsigned left = 0;
+            float poi[kBatch], poj[kBatch], pwi[kBatch], pwj[kBatch], pu[kBatch];
+            auto fetch = [&]() {
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    while (!left && q < kGroup / 32) left = __shfl_sync(0xffffffffu, mine, ++q);
+                    ne[k] = left ? 32 * q + __ffs(left) - 1 : -1;
+                    left &= left - 1;
+                    pu[k] = ne[k] >= 0 ? best_so_far(best + e0 + ne[k]) : 0.0f;
+                    const bool on = ne[k] >= 0 && lane < half;
+                    const size_t at = (size_t)(e0 + (on ? ne[k] : 0)) * ntf + (on ? lane : 0);
+                    poi[k] = __ldg(obs + at);
+                    poj[k] = __ldg(obs + at + half);
+                    pwi[k] = on ? __ldg(wts + at) : 0.0f;
+                    pwj[k] = __ldg(wts + at + half);
+                }
+            };
+            fetch();
+            block_arrived();
+            float sumT = 0.0f;
+#pragma unroll 8
+            for (int i = 0; i < ntf; ++i) sumT += fabsf(s_t[32 * i + lane]);
+            while (ne[0] >= 0) {
+                __syncwarp();
+                float v[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) v[k] = pwi[k] > 0.0f && pwj[k] > 0.0f ? poi[k] - poj[k] : NONE;
+                if (lane < np) s_ev[lane] = make_float4(v[0], v[1], v[2], v[3]);
+                __syncwarp();
+                int e[kBatch];
+                bool x[kBatch];
+                float thr[kBatch], la[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    x[k] = ne[k] >= 0;
+                    e[k] = x[k] ? ne[k] : ne[0];
+                    thr[k] = signbit(pu[k]) ? INF
+                                            : fmaf(pu[k] / s_wv[e[k]], 1.0f + 1.0f / 1048576, kSlackL1 * (sumT + s_o[e[k]]));
+                    la[k] = 0.0f;
+                }
+                fetch();
+#pragma unroll 1
+                for (int l = 0; l < np; l += 8) {
+#pragma unroll
+                    for (int i = l; i < l + 8; ++i) {
+                        if (i >= half) break;
+                        const float t = s_t[32 * i + lane] - s_t[32 * (i + half) + lane];
+                        const float4 v = s_ev[i];
+                        la[0] += fmaxf(fabsf(v.x - t), 0.0f);
+                        la[1] += fmaxf(fabsf(v.y - t), 0.0f);
+                        la[2] += fmaxf(fabsf(v.z - t), 0.0f);
+                        la[3] += fmaxf(fabsf(v.w - t), 0.0f);
+                    }
+                    bool any = false;
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        x[k] = __any_sync(0xffffffffu, in && x[k] && !(la[k] > thr[k]));
+                        any |= x[k];
+                    }
+                    if (!any) break;
+                }
+#pragma unroll 1
+                for (int k = 0; k < kBatch; ++k) {
+                    if (!(k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3])) continue;
+                    const int ek = k == 0 ? e[0] : k == 1 ? e[1] : k == 2 ? e[2] : e[3];
+                    __syncwarp();
+                    for (int i = lane; i < ntf; i += 32)
+                        s_ow[i] = make_float2(__ldg(obs + (size_t)(e0 + ek) * ntf + i), __ldg(wts + (size_t)(e0 + ek) * ntf + i));
+                    __syncwarp();
+                    float r[N];
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        r[i] = INF;
+                        if (i < ntf) {
+                            const float2 ow = s_ow[i];
+                            if (ow.y > 0.0f) r[i] = ow.x - s_t[32 * i + lane];
+                        }
+                    }
+                    const int m = s_n[ek];
+                    const float obj = l1_sorted_misfit<N>(r, m) * s_wv[ek];
+                    const unsigned long long key = warp_min((in && m > 0) ? pack_key(obj, g) : ~0ull);
+                    if (lane == 0) atomicMin(best + e0 + ek, key);
+                }
+            }
+        }
+    }
+}
+
+/* One or two launches, as launch_l2_search. */
+/* Where blocks pay, as for L2; the point bound is dear here, so earlier.  By
+ * points / by blocks, us: 100 events x 99e3 points x 20 tables 206 / 155, 30
+ * events x 144e3 x 20 128 / 128, 10 x 99e3 x 20 81 / 99; above 32 tables (64
+ * residuals to sort, two CTAs to an SM) 100 x 144e3 x 60 430 / 468, 20 x 541e3
+ * x 60 336 / 348, 64 x 541e3 x 60 679 / 542. */
+inline int l1_block_events(int ntf) { return ntf <= 32 ? 32 : 64; }
+inline int l1_block_points(int ntf) { return ntf <= 32 ? 1 << 16 : 1 << 18; }
+
+
+template <int N>
+cudaError_t launch_l1_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
                       unsigned long long *best, cudaStream_t s)
 {
     const long long ctas = (ngrd + (long long)kThreads - 1) / kThreads;
-    const dim3 grid((unsigned)ctas, event_split(ctas, nev));
+    int chunk;
+    const dim3 grid = point_grid(ctas, nev, &chunk);
     if (ngrd < kBoundPoints) {
-        l1_search_kernel<N, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, best);
-        return;
+        l1_search_kernel<N, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, best);
+        return cudaSuccess;
     }
     const long long cs = ((ngrd + kSample - 1) / kSample + (long long)kThreads - 1) / kThreads;
-    l1_search_kernel<N, false><<<dim3((unsigned)cs, event_split(cs, nev)), kThreads, 0, s>>>(
-        ngrd, ldgrd, ntf, kSample, tables, nev, obs, wts, best);
-    l1_search_kernel<N, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, obs, wts, best);
+    int schunk;
+    const dim3 sgrid = point_grid(cs, nev, &schunk);
+    l1_search_kernel<N, false><<<sgrid, kThreads, 0, s>>>(
+        ngrd, ldgrd, ntf, kSample, tables, nev, schunk, obs, wts, best);
+    if (nev < l1_block_events(ntf) || ngrd < l1_block_points(ntf)) {
+        l1_search_kernel<N, true><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, best);
+        return cudaSuccess;
+    }
+    int group;
+    const dim3 gb = block_grid(ngrd, nev, &group);
+    const size_t smem = l1_block_smem(ntf);
+    const cudaError_t ea = cudaFuncSetAttribute(l1_block_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ea != cudaSuccess) return ea;
+    l1_block_kernel<N><<<gb, kBlkThreads, smem, s>>>(ngrd, ldgrd, ntf, tables, nev, group, obs, wts, best);
+    return cudaSuccess;
 }
 
 /* FP64 median and misfit at the chosen point from the FP64 picks
@@ -945,9 +1217,9 @@ extern "C" int fk_locate_l1_exact(int ngrd, int ldgrd, int ntf, const float *tab
     if (nev <= 0) return 0;
     if (ntf < 1 || ntf > kMaxTf) return (int)cudaErrorInvalidValue;
     l1_init_kernel<<<(nev + 255) / 256, 256, 0, s>>>(nev, scratch);
-    if (ntf <= 16) launch_l1_search<16>(ngrd, ldgrd, ntf, tables, nev, obs, wts, scratch, s);
-    else if (ntf <= 32) launch_l1_search<32>(ngrd, ldgrd, ntf, tables, nev, obs, wts, scratch, s);
-    else launch_l1_search<64>(ngrd, ldgrd, ntf, tables, nev, obs, wts, scratch, s);
+    auto *search = ntf <= 16 ? launch_l1_search<16> : ntf <= 32 ? launch_l1_search<32> : launch_l1_search<64>;
+    const cudaError_t e = search(ngrd, ldgrd, ntf, tables, nev, obs, wts, scratch, s);
+    if (e != cudaSuccess) return (int)e;
     l1_at_opt_kernel<<<(nev + 127) / 128, 128, 0, s>>>(ldgrd, ntf, tables, nev, obs64, wts64, scratch, out_idx,
                                                        out_t0, out_obj);
     return (int)cudaGetLastError();

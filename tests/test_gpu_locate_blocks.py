@@ -2,7 +2,7 @@
 optimum, origin time and misfit equal, bit for bit, those of the same events
 searched in smaller groups (each point bounded by itself) and the oracle's, at
 the edges of blocks, of a thread block's 1024 points, of the table widths and of
-the event groups."""
+the event groups.  L1: equal to the search in smaller groups."""
 import numpy as np
 import pytest
 
@@ -41,4 +41,35 @@ def test_blocks_match_points_and_oracle_bitwise(fk, ntf, ngrd, nev, kind):
             np.testing.assert_array_equal(a[e0:e0 + 150], np.array(b))
     for e in (0, nev // 2, nev - 1):
         assert tuple(v[e] for v in got) == _oracle(tables, picks[e], wts[e]), e
+    loc.finalize()
+
+
+@pytest.mark.parametrize("ntf,ngrd,nev", [(1, 1 << 16, 32), (2, (1 << 16) + 1, 33), (17, (1 << 16) + 1055, 64), (32, 1 << 16, 300),
+                                          (33, 1 << 18, 64), (64, (1 << 18) + 31, 65)])
+@pytest.mark.parametrize("kind", ["times", "random"])
+def test_l1_blocks_match_points(fk, ntf, ngrd, nev, kind):
+    rng = np.random.default_rng(ntf * 10 + nev)
+    if kind == "times":
+        n = ngrd // 4096 + 1
+        tables = np.ascontiguousarray(station_tables(64, 64, n, 50.0, ntf, seed=ntf)[:, :ngrd])
+    else:
+        tables = rng.uniform(0.5, 12.0, (ntf, ngrd)).astype(np.float32)
+    _, picks = synthetic_events(tables, nev, seed=ntf + 2)
+    wts = np.full(picks.shape, 0.5)
+    wts[rng.random(picks.shape) < 0.15] = 0.0
+    wts[:, 0] = 0.5
+    if ntf > 3:                   # an unreachable table, unused by all events
+        tables[2, : ngrd // 2] = np.inf
+        wts[:, 2] = 0.0
+    loc = fk.Locator(nev, ntf, ngrd)
+    for k in range(ntf):
+        loc.setTravelTimeField32f(k + 1, tables[k])
+    for e in range(nev):
+        loc.setObservation(e + 1, np.arange(1, ntf + 1), picks[e], wts[e])
+    loc.setNorm(1)
+    got = [np.array(v) for v in loc.locateEvents(np.arange(1, nev + 1))]
+    for e0 in range(0, nev, 30):
+        few = loc.locateEvents(np.arange(e0 + 1, min(nev, e0 + 30) + 1))
+        for a, b in zip(got, few):
+            np.testing.assert_array_equal(a[e0:e0 + 30], np.array(b))
     loc.finalize()
