@@ -180,7 +180,10 @@ static void set_work(fk_work2d_t *w, int isrc, double *tt)
 }
 
 /* Solve n work items of one grid (g, also at grid_dev): by the diagonal walk
- * where it applies, in pieces of at most 1 GiB of field copies. */
+ * where it applies, in pieces of at most 4 GiB of field copies (1 GiB if
+ * memory is short).  A piece takes its chain of steps however few SMs it fills,
+ * so pieces that do not hold all sources hold whole waves: 148 sources on 400 x
+ * 500 in pieces of 144 and 4 took 10.2 ms, in one 6.0. */
 static int run_solve(int fsm, const fk_grid2d_t *g, const fk_work2d_t *work, fk_result3d_t *res, int n, cudaStream_t s,
                      const char *who)
 {
@@ -188,15 +191,29 @@ static int run_solve(int fsm, const fk_grid2d_t *g, const fk_work2d_t *work, fk_
     if (!fk2d_diag_bytes(g->nz, g->nx, &model, &source))
         /* solver2D.F90:935-946: the reference's test never stops early */
         return fk2d_solve(fsm, S2.grid_dev, work, res, n, g->nx, g->nz, S2.eps, S2.nsweep, -1.0, 0, s);
-    size_t most = ((size_t)1 << 30) / source;
-    if (most < 1) most = 1;
-    if (most > (size_t)n) most = (size_t)n;
-    const size_t need = model + most * source;
-    if (need > S2.diag_cap) {
+    size_t most = 0;
+    for (size_t limit = (size_t)4 << 30;; limit /= 2) {
+        most = limit / source;
+        if (most < (size_t)n && most > 148) most -= most % 148;   /* the SMs */
+        if (most < 1) most = 1;
+        if (most > (size_t)n) most = (size_t)n;
+        const size_t need = model + most * source;
+        if (need <= S2.diag_cap) break;
         fk_dfree(S2.diag);
-        S2.diag = fk_dalloc(need, who);
-        S2.diag_cap = S2.diag ? need : 0;
-        if (!S2.diag) return (int)cudaErrorMemoryAllocation;
+        S2.diag = NULL;
+        S2.diag_cap = 0;
+        if (limit > (size_t)1 << 30) {
+            if (cudaMalloc(&S2.diag, need) != cudaSuccess) {
+                (void)cudaGetLastError();
+                S2.diag = NULL;
+                continue;
+            }
+        } else {
+            S2.diag = fk_dalloc(need, who);
+            if (!S2.diag) return (int)cudaErrorMemoryAllocation;
+        }
+        S2.diag_cap = need;
+        break;
     }
     int e = 0;
     for (int i = 0; !e && i < n; i += (int)most) {

@@ -711,11 +711,16 @@ extern "C" int fk2d_solve_diag(const fk_grid2d_t *grid, const fk_work2d_t *work,
     diag_fill_kernel<<<(unsigned)(n2 / 512 + 1 < 148 * 16 ? n2 / 512 + 1 : 148 * 16), 256, 0, stream>>>(
         (double2 *)dg.field, n2);
     /* 256 sources on 151 x 301: 3.0 ms with two CTAs to an SM (102 registers),
-     * 4.2 with one (128); one source on 201 x 201 is 2 % faster with 176
-     * registers than with 128 */
+     * 4.2 with one (128); 200 on 200 x 360 4.3 and 5.2 (80 registers), 256 on
+     * 250 x 400 6.2 and 6.9 (72), but 256 on 400 x 500 11.5 and 10.7 (64); one
+     * source on 201 x 201 is 2 % faster with 176 registers than with 128 */
     const bool share = nwork > 148;
-    auto *kernel = dg.pitch <= 256 ? (share ? diag_solve_kernel<256, 2> : diag_solve_kernel<256, 1>)
-                                   : (share && dg.pitch <= 320 ? diag_solve_kernel<320, 2> : diag_solve_kernel<kDiagCols, 1>);
+    auto *kernel = dg.pitch <= 256   ? (share ? diag_solve_kernel<256, 2> : diag_solve_kernel<256, 1>)
+                   : !share          ? diag_solve_kernel<kDiagCols, 1>
+                   : dg.pitch <= 320 ? diag_solve_kernel<320, 2>
+                   : dg.pitch <= 384 ? diag_solve_kernel<384, 2>
+                   : dg.pitch <= 448 ? diag_solve_kernel<448, 2>
+                                     : diag_solve_kernel<kDiagCols, 1>;
     kernel<<<nwork, dg.pitch, 0, stream>>>(g, work, results, dg, eps, nsweep);
     for (int w0 = 0; w0 < nwork; w0 += 65535) {
         Diag2 d1 = dg;
