@@ -75,9 +75,14 @@ constexpr float kSlackO2 = 1.0f / 1048576; /* 2^-20 = 16 e */
  * tables while it runs over the events blockIdx.y, + gridDim.y, ... (in
  * chunks of kEvChunk).  BOUND: rule out by the bound first, level by level
  * (the sums carry on), while any of the warp's points survives.  The bound
- * costs 3 packed operations and one 16-byte shared-memory broadcast a pick. */
+ * costs 3 packed operations and one 16-byte shared-memory broadcast a pick.
+ * The points are loaded, then evaluated, and the warps of the other CTAs of an
+ * SM fill the gaps: 8, 4, 4 and 3 CTAs for 16, 32, 48 and 64 tables held.  One
+ * event x 48 tables x 1.31e6 points 101 us a call with 48 tables held (4 CTAs),
+ * 114 with 64 (3); 100 events x 14 x 542e3 183 us with 8 CTAs, 205 with 4; 40 x
+ * 20 x 1.09e6 228 us with 4, 250 with 6. */
 template <int NTF, bool BOUND>
-__global__ void __launch_bounds__(kThreads, NTF == 64 ? 3 : 4)
+__global__ void __launch_bounds__(kThreads, NTF == 64 ? 3 : NTF == 16 ? 8 : 4)
 l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restrict__ tables, int nev, int chunk,
                  const float *__restrict__ obs, const float *__restrict__ wts,
                  const float *__restrict__ xnorm, unsigned long long *best)
@@ -670,7 +675,10 @@ extern "C" int fk_locate_l2_exact(int ngrd, int ldgrd, int ntf, const float *tab
     unsigned long long *best = (unsigned long long *)scratch;
     float *xn = (float *)(best + nev);
     xnorm_kernel<<<(nev + 127) / 128, 128, 0, s>>>(nev, ntf, wts, xn, best);
-    auto *search = ntf <= 16 ? launch_l2_search<16> : ntf <= 32 ? launch_l2_search<32> : launch_l2_search<64>;
+    auto *search = ntf <= 16   ? launch_l2_search<16>
+                   : ntf <= 32 ? launch_l2_search<32>
+                   : ntf <= 48 ? launch_l2_search<48>
+                               : launch_l2_search<64>;
     const cudaError_t e = search(ngrd, ldgrd, ntf, tables, nev, obs, wts, xn, best, s);
     if (e != cudaSuccess) return (int)e;
     l2_at_opt_kernel<<<(nev + 3) / 4, 128, 0, s>>>(ldgrd, ntf, tables, nev, obs, wts, xn, best, out_idx, out_t0,

@@ -73,3 +73,23 @@ def test_l1_blocks_match_points(fk, ntf, ngrd, nev, kind):
         for a, b in zip(got, few):
             np.testing.assert_array_equal(a[e0:e0 + 30], np.array(b))
     loc.finalize()
+
+
+@pytest.mark.parametrize("ntf", [15, 16, 32, 47, 48])
+@pytest.mark.parametrize("nev,ngrd", [(1, 4111), (8, 4096), (21, 4225)])
+def test_table_widths_match_oracle_bitwise(fk, ntf, nev, ngrd):
+    tables = np.ascontiguousarray(station_tables(16, 16, 17, 100.0, ntf, seed=ntf)[:, :ngrd])
+    _, picks = synthetic_events(tables, nev, seed=ntf + 1)
+    rng = np.random.default_rng(ntf + nev)
+    wts = rng.choice([1.0, 0.75, 0.5, 0.25], picks.shape)
+    wts[rng.random(picks.shape) < 0.15] = 0.0
+    wts[:, 0] = 1.0
+    loc = fk.Locator(nev, ntf, tables.shape[1])
+    for k in range(ntf):
+        loc.setTravelTimeField32f(k + 1, tables[k])
+    for e in range(nev):
+        loc.setObservation(e + 1, np.arange(1, ntf + 1), picks[e], wts[e])
+    got = loc.locateEvents(np.arange(1, nev + 1))
+    for e in range(nev):
+        assert tuple(v[e] for v in got) == _oracle(tables, picks[e], wts[e]), e
+    loc.finalize()
