@@ -534,50 +534,76 @@ l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
     }
 }
 
-/* t0 and obj at the optimum, same arithmetic: a warp per event fetches its
- * 64 terms at once, one lane adds them in order. */
+/* Sum of kMaxTf values in shared memory, in order (16-byte loads a few ahead of
+ * the chain of additions). */
+__device__ __forceinline__ float ordered_sum(const float *v, int n)
+{
+    float s = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < n; i += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(v + i);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, q.x), q.y), q.z), q.w);
+    }
+    return s;
+}
+
+/* t0 and obj at the optimum, same arithmetic: a warp per event forms its terms,
+ * two a lane, and adds them in order; a skipped pick's is +0, which leaves a
+ * sum that started at +0 as it is.  With one lane forming and adding all terms
+ * one event took 7.5 us, the normaliser below 4.5 (one thread an event, loads in
+ * its chain): together 4 to 6 us of a call (45 tables x 542e3 points 73.7 -> 67.4). */
 __global__ void __launch_bounds__(128)
 l2_at_opt_kernel(int ldgrd, int ntf, const float *__restrict__ tables, int nev, const float *__restrict__ obs,
                  const float *__restrict__ wts, const float *__restrict__ xnorm,
                  const unsigned long long *__restrict__ best, int *out_idx, float *out_t0, float *out_obj)
 {
-    __shared__ float s_o[4][kMaxTf], s_w[4][kMaxTf], s_t[4][kMaxTf];
+    __shared__ __align__(16) float s_term[4][2][kMaxTf];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.x * 4 + warp;
     if (e >= nev) return;
     const int g = (int)(best[e] & 0xffffffffu);
-    for (int i = lane; i < ntf; i += 32) {
-        s_o[warp][i] = obs[(size_t)e * ntf + i];
-        s_w[warp][i] = wts[(size_t)e * ntf + i];
-        s_t[warp][i] = tables[(size_t)i * ldgrd + g];
+    const float xn = xnorm[e];
+    float o[kMaxTf / 32], w[kMaxTf / 32], T[kMaxTf / 32];
+#pragma unroll
+    for (int h = 0; h < kMaxTf / 32; ++h) {
+        const int i = 32 * h + lane;
+        const bool in = i < ntf;
+        o[h] = in ? obs[(size_t)e * ntf + i] : 0.0f;
+        w[h] = in ? wts[(size_t)e * ntf + i] : 0.0f;
+        T[h] = in ? tables[(size_t)i * ldgrd + g] : 0.0f;
+        s_term[warp][0][i] = w[h] > 0.0f ? __fmul_rn(w[h], __fmul_rn(xn, __fsub_rn(o[h], T[h]))) : 0.0f;
     }
     __syncwarp();
-    if (lane != 0) return;
-    const float *o = s_o[warp], *w = s_w[warp], *T = s_t[warp];
-    const float xn = xnorm[e];
-    float t0 = 0.0f;
-    for (int i = 0; i < ntf; ++i)
-        if (w[i] > 0.0f) t0 = __fadd_rn(t0, __fmul_rn(w[i], __fmul_rn(xn, __fsub_rn(o[i], T[i]))));
-    float obj = 0.0f;
-    for (int i = 0; i < ntf; ++i)
-        if (w[i] > 0.0f) {
-            const float res = __fmul_rn(__fmul_rn(0.70710677f, w[i]), __fsub_rn(o[i], __fadd_rn(T[i], t0)));
-            obj = __fadd_rn(obj, __fmul_rn(res, res));
-        }
-    out_idx[e] = g;
-    out_t0[e] = t0;
-    out_obj[e] = obj;
+    const int n4 = (ntf + 3) / 4 * 4;
+    const float t0 = ordered_sum(s_term[warp][0], n4);
+#pragma unroll
+    for (int h = 0; h < kMaxTf / 32; ++h) {
+        const float res = __fmul_rn(__fmul_rn(0.70710677f, w[h]), __fsub_rn(o[h], __fadd_rn(T[h], t0)));
+        s_term[warp][1][32 * h + lane] = w[h] > 0.0f ? __fmul_rn(res, res) : 0.0f;
+    }
+    __syncwarp();
+    const float obj = ordered_sum(s_term[warp][1], n4);
+    if (lane == 0) {
+        out_idx[e] = g;
+        out_t0[e] = t0;
+        out_obj[e] = obj;
+    }
 }
 
-__global__ void xnorm_kernel(int nev, int ntf, const float *__restrict__ wts, float *xnorm,
-                             unsigned long long *best)
+/* 1 / SUM over the padded weight row, in order; a warp per event. */
+__global__ void __launch_bounds__(128) xnorm_kernel(int nev, int ntf, const float *__restrict__ wts, float *xnorm,
+                                                    unsigned long long *best)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ __align__(16) float s_w[4][kMaxTf];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e = blockIdx.x * 4 + warp;
     if (e >= nev) return;
-    float s = 0.0f; /* SUM over the padded weight row, in order */
-    for (int i = 0; i < ntf; ++i) s = __fadd_rn(s, wts[(size_t)e * ntf + i]);
-    xnorm[e] = __fdiv_rn(1.0f, s);
-    best[e] = ~0ull;
+    for (int i = lane; i < kMaxTf; i += 32) s_w[warp][i] = i < ntf ? wts[(size_t)e * ntf + i] : 0.0f;
+    __syncwarp();
+    if (lane == 0) {
+        xnorm[e] = __fdiv_rn(1.0f, ordered_sum(s_w[warp], (ntf + 3) / 4 * 4));
+        best[e] = ~0ull;
+    }
 }
 
 /* Searches the points in one launch, or in two: fewer than kBoundEvents
@@ -674,7 +700,7 @@ extern "C" int fk_locate_l2_exact(int ngrd, int ldgrd, int ntf, const float *tab
     if (scratch_bytes < fk_locate_l2_exact_scratch(ngrd, nev)) return (int)cudaErrorInvalidValue;
     unsigned long long *best = (unsigned long long *)scratch;
     float *xn = (float *)(best + nev);
-    xnorm_kernel<<<(nev + 127) / 128, 128, 0, s>>>(nev, ntf, wts, xn, best);
+    xnorm_kernel<<<(nev + 3) / 4, 128, 0, s>>>(nev, ntf, wts, xn, best);
     auto *search = ntf <= 16   ? launch_l2_search<16>
                    : ntf <= 32 ? launch_l2_search<32>
                    : ntf <= 48 ? launch_l2_search<48>
