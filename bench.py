@@ -610,8 +610,8 @@ def bench_locate(fk, b, grids, stream, steps, nev=LOC_NEV, igrid=LOC_GRID, sur_s
                                  "tflops": flops_row * ncoarse * NSRC / t_bd / 1e12}},
             "l1_exhaustive": {"events_per_s": len(l1_sample) / (l1_ms * 1e-3), "ms": l1_ms,
                               "sample_events": len(l1_sample),
-                              "method": "median origin time, 64-key bitonic sort per grid point, FP32 ranking, "
-                                        "FP64 optimum"},
+                              "method": "median origin time, points ruled out by pairs of picks or sorted (64-key "
+                                        "bitonic network), FP32 ranking, FP64 optimum"},
             "exact_fp32": {"events_per_s": len(sample) / (ex_ms * 1e-3), "ms": ex_ms,
                            "sample_events": len(sample)},
             "hypocentre_agreement_tc_vs_exact": agree}

@@ -550,8 +550,8 @@ __device__ __forceinline__ float ordered_sum(const float *v, int n)
 /* t0 and obj at the optimum, same arithmetic: a warp per event forms its terms,
  * two a lane, and adds them in order; a skipped pick's is +0, which leaves a
  * sum that started at +0 as it is.  With one lane forming and adding all terms
- * one event took 7.5 us, the normaliser below 4.5 (one thread an event, loads in
- * its chain): together 4 to 6 us of a call (45 tables x 542e3 points 73.7 -> 67.4). */
+ * the kernel took 7.5 us for one event, so 5.6 (one event x 45 tables x 542e3
+ * points 73.7 -> 67.4 us a call, the weights' sum below included). */
 __global__ void __launch_bounds__(128)
 l2_at_opt_kernel(int ldgrd, int ntf, const float *__restrict__ tables, int nev, const float *__restrict__ obs,
                  const float *__restrict__ wts, const float *__restrict__ xnorm,
