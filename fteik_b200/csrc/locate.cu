@@ -675,7 +675,9 @@ cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, 
     const dim3 gb = block_grid(ngrd, nev, &group);
     const size_t smem = block_smem(ntf);
     auto *kernel = ntf <= 48 ? l2_block_kernel<3> : l2_block_kernel<2>;
-    const cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    /* the limit for the widest tables it serves: calls of other threads may set it too */
+    const cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)block_smem(ntf <= 48 ? 48 : kMaxTf));
     if (ea != cudaSuccess) return ea;
     kernel<<<gb, kBlkThreads, smem, s>>>(
         ngrd, ldgrd, ntf, tables, nev, group, obs, wts, xn, best);
@@ -1196,7 +1198,8 @@ cudaError_t launch_l1_search(int ngrd, int ldgrd, int ntf, const float *tables, 
     int group;
     const dim3 gb = block_grid(ngrd, nev, &group);
     const size_t smem = l1_block_smem(ntf);
-    const cudaError_t ea = cudaFuncSetAttribute(l1_block_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t ea =
+        cudaFuncSetAttribute(l1_block_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l1_block_smem(N));
     if (ea != cudaSuccess) return ea;
     l1_block_kernel<N><<<gb, kBlkThreads, smem, s>>>(ngrd, ldgrd, ntf, tables, nev, group, obs, wts, best);
     return cudaSuccess;
