@@ -442,9 +442,10 @@ static int build_work(const char *who)
  * kernel for both, takes their place if it beats the two together.  Every candidate is run
  * twice and timed by its faster run.  Every configuration gives the same
  * fields bit for bit, so the search changes only the time.  The choice is
- * kept per work list (grid shapes, sources per grid, precision, passes) in
- * memory and, when FTEIK_B200_TUNE_CACHE names a file, in that file, so
- * later processes skip the search. */
+ * kept per work list (grid shapes, sources per grid, precision, passes) and
+ * knobs, set ones and open ones (the search they leave differs), in memory
+ * and, when FTEIK_B200_TUNE_CACHE names a file, in that file, so later
+ * processes skip the search. */
 #define TILE_LAUNCHES 8
 
 static void tune_apply(const int t[7])
@@ -461,6 +462,7 @@ static void tune_apply(const int t[7])
 
 static void tune_key(char *key, size_t cap)
 {
+    const fk_slabcfg_t k = fk_slabcfg();
     struct cudaDeviceProp prop;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -468,8 +470,9 @@ static void tune_key(char *key, size_t cap)
         prop.name[0] = 0;
         prop.multiProcessorCount = 0;
     }
-    size_t o = (size_t)snprintf(key, cap, "%s|sm%d|p%d|n%d|c%d:%d|", prop.name, prop.multiProcessorCount,
-                                SB.precision, SB.nsweep, SB.conv_tol >= 0.0, SB.max_pass);
+    size_t o = (size_t)snprintf(key, cap, "%s|sm%d|p%d|n%d|c%d:%d|v7|k%d,%d,%d,%d|", prop.name,
+                                prop.multiProcessorCount, SB.precision, SB.nsweep, SB.conv_tol >= 0.0, SB.max_pass,
+                                k.staged, k.pairs, k.progress, k.blocks_per_sm);   /* v7: seven values a line */
     for (int i = 0; i < SB.ngrid && o < cap; i++)
         o += (size_t)snprintf(key + o, cap - o, "%dx%dx%dx%d;", SB.g[i].nz, SB.g[i].nx, SB.g[i].ny, SB.g[i].nsrc);
     for (char *c = key; *c; c++)
@@ -492,8 +495,8 @@ static int tune_lookup(const char *key, int t[7])
     char line[700], k[600];
     int found = 0;
     while (fgets(line, sizeof(line), f)) {
-        int v[7] = {0};   /* lines written before the tile schedule have six values */
-        if (sscanf(line, "%599s %d %d %d %d %d %d %d", k, &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6]) >= 7 &&
+        int v[7];
+        if (sscanf(line, "%599s %d %d %d %d %d %d %d", k, &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6]) == 8 &&
             strcmp(k, key) == 0) {
             memcpy(t, v, sizeof(v));
             found = 1;    /* the last line for a key wins */
@@ -561,8 +564,6 @@ static int tune(const char *who)
     const bool tiles = cfg.staged < 0 && cfg.pairs < 0 && cfg.progress < 0 && cfg.blocks_per_sm < 0;
     const int conv = SB.conv_tol >= 0.0 && SB.max_pass > 0;
     if (tune_lookup(key, t)) {
-        /* the knobs left open are part of the choice: a set one rules out the tiles */
-        if (!tiles) t[6] = 0;
         if (t[6] && fk_slabplan_tiles(&SB.plan, SB.precision, conv, who)) return 1;
         tune_apply(t);
         return 0;

@@ -382,7 +382,7 @@ void fteik_b200_batch3d_getTravelTimes64f(int igrid, int nval, double ttr[],
                                           int *ierr);
 /* The launch configuration the batch runs (see fteik_b200_setSlabConfig):
  * knobs left at -1 are chosen by timing the candidates on the first solve of
- * a new work list (grid shapes, sources per grid, precision, passes); the
+ * a new work list (grid shapes, sources per grid, precision, passes, knobs); the
  * initialisation kernel takes its own blocks per SM and source pairing
  * (initPairs: two sources per thread over the union of their boxes).  The
  * choice is remembered in the process and, when the environment variable
