@@ -30,7 +30,7 @@ static struct {
     int rec_cap;
     double *gx, *gz;      /* device [ngrd] gradient of the current field */
     void *diag;           /* diagonal walk's scratch (fk2d_solve_diag) */
-    size_t diag_cap;
+    size_t diag_cap, diag_limit;   /* limit: field copies of a piece (0: not chosen) */
     bool have_grad;
 } S2;
 
@@ -179,47 +179,50 @@ static void set_work(fk_work2d_t *w, int isrc, double *tt)
     w->tt = tt;
 }
 
-/* Solve n work items of one grid (g, also at grid_dev): by the diagonal walk
- * where it applies, in pieces of at most 4 GiB of field copies (1 GiB if
- * memory is short).  A piece takes its chain of steps however few SMs it fills,
- * so pieces that do not hold all sources hold whole waves: 148 sources on 400 x
- * 500 in pieces of 144 and 4 took 10.2 ms, in one 6.0. */
-static int run_solve(int fsm, const fk_grid2d_t *g, const fk_work2d_t *work, fk_result3d_t *res, int n, cudaStream_t s,
-                     const char *who)
+/* Device scratch of the diagonal walk: the sources of a piece, 0 if there is not
+ * enough memory.  A piece holds at most 4 GiB of field copies, 2 or 1 GiB once
+ * more could not be had, and the scratch, which stays until the solver is freed,
+ * at most half of the device memory that was free (the rest is for the arrays
+ * that later calls allocate).  A piece takes its chain of steps however few SMs
+ * it fills, so pieces that do not hold all sources hold whole waves: 148 sources
+ * on 400 x 500 in pieces of 144 and 4 took 10.2 ms, in one 6.0. */
+static int diag_scratch(size_t model, size_t source, int n)
 {
-    size_t model, source;
-    if (!fk2d_diag_bytes(g->nz, g->nx, &model, &source))
-        /* solver2D.F90:935-946: the reference's test never stops early */
-        return fk2d_solve(fsm, S2.grid_dev, work, res, n, g->nx, g->nz, S2.eps, S2.nsweep, -1.0, 0, s);
-    size_t most = 0;
-    for (size_t limit = (size_t)4 << 30;; limit /= 2) {
-        most = limit / source;
+    const size_t least = (size_t)1 << 30;
+    if (!S2.diag_limit) S2.diag_limit = 4 * least;
+    for (;; S2.diag_limit /= 2) {
+        size_t most = S2.diag_limit / source, room = 0, total;
         if (most < (size_t)n && most > 148) most -= most % 148;   /* the SMs */
         if (most < 1) most = 1;
         if (most > (size_t)n) most = (size_t)n;
         const size_t need = model + most * source;
-        if (need <= S2.diag_cap) break;
+        if (need <= S2.diag_cap) return (int)most;
         fk_dfree(S2.diag);
         S2.diag = NULL;
         S2.diag_cap = 0;
-        if (limit > (size_t)1 << 30) {
-            if (cudaMalloc(&S2.diag, need) != cudaSuccess) {
-                (void)cudaGetLastError();
-                S2.diag = NULL;
-                continue;
-            }
-        } else {
-            S2.diag = fk_dalloc(need, who);
-            if (!S2.diag) return (int)cudaErrorMemoryAllocation;
+        if (cudaMemGetInfo(&room, &total) == cudaSuccess && need <= room / 2 &&
+            cudaMalloc(&S2.diag, need) == cudaSuccess) {
+            S2.diag_cap = need;
+            return (int)most;
         }
-        S2.diag_cap = need;
-        break;
+        (void)cudaGetLastError();
+        S2.diag = NULL;
+        if (S2.diag_limit <= least) return 0;
     }
+}
+
+/* Solve n work items of one grid (g, also at grid_dev): by the diagonal walk
+ * where it applies and its scratch can be had, else in place. */
+static int run_solve(int fsm, const fk_grid2d_t *g, const fk_work2d_t *work, fk_result3d_t *res, int n, cudaStream_t s)
+{
+    size_t model, source;
+    const int most = fk2d_diag_bytes(g->nz, g->nx, &model, &source) ? diag_scratch(model, source, n) : 0;
+    if (!most)
+        /* solver2D.F90:935-946: the reference's test never stops early */
+        return fk2d_solve(fsm, S2.grid_dev, work, res, n, g->nx, g->nz, S2.eps, S2.nsweep, -1.0, 0, s);
     int e = 0;
-    for (int i = 0; !e && i < n; i += (int)most) {
-        const int m = n - i < (int)most ? n - i : (int)most;
-        e = fk2d_solve_diag(g, work + i, res + i, m, S2.eps, S2.nsweep, S2.diag, i == 0, s);
-    }
+    for (int i = 0; !e && i < n; i += most)
+        e = fk2d_solve_diag(g, work + i, res + i, n - i < most ? n - i : most, S2.eps, S2.nsweep, S2.diag, i == 0, s);
     return e;
 }
 
@@ -248,7 +251,7 @@ static int solve_one(int isrc, int fsm, const char *who)
     fk_result3d_t res;
     int e = (int)cudaMemcpyAsync(S2.grid_dev, &g, sizeof(g), cudaMemcpyHostToDevice, s);
     if (!e) e = (int)cudaMemcpyAsync(S2.work_dev, &w, sizeof(w), cudaMemcpyHostToDevice, s);
-    if (!e) e = run_solve(fsm, &g, S2.work_dev, S2.res_dev, 1, s, who);
+    if (!e) e = run_solve(fsm, &g, S2.work_dev, S2.res_dev, 1, s);
     if (!e) e = (int)cudaMemcpyAsync(&res, S2.res_dev, sizeof(res), cudaMemcpyDeviceToHost, s);
     if (!e) e = (int)cudaStreamSynchronize(s);
     if (fk_check(e, who) || res.status) return 1;
@@ -346,7 +349,7 @@ static int solve_chunks(const char *who)
         }
         e = (int)cudaMemcpyAsync(S2.work_all, w, sizeof(fk_work2d_t) * (size_t)n, cudaMemcpyHostToDevice, s);
         if (!e) e = (int)cudaMemcpyAsync(S2.fptr_dev, fp, sizeof(void *) * (size_t)n, cudaMemcpyHostToDevice, s);
-        if (!e) e = run_solve(0, &g, S2.work_all, S2.res_all, n, s, who);
+        if (!e) e = run_solve(0, &g, S2.work_all, S2.res_all, n, s);
         if (!e && nrec > 0)
             e = fk_receivers_batch2d(nx, zp, fk_model.dz, fk_model.dx, S2.fptr_dev, n, nrec, fk_receiver.ri_dev,
                                      fk_receiver.rd_dev, S2.rec_all, s);

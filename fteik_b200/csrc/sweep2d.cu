@@ -4,7 +4,8 @@
  * solveSourceFSM (solver2D.F90:1042-1280), in FP64.
  *
  * Grids up to 512 columns take the diagonal walk (second half of the file);
- * wider ones, and solves to convergence, the walk in place:
+ * wider ones, solves to convergence, and those for whose scratch the device has
+ * no memory left, the walk in place:
  *
  * One CTA owns one (grid, source).  Thread t owns the logical x columns
  * b NT + t (b = 0, 1, ...: column blocks of NT <= 512 threads) and walks
