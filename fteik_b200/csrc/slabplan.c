@@ -155,7 +155,7 @@ int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char
     const int n = pl->nwork, nz = pl->dev.max_nz;
     const int cap = fk3d_tile_capacity(precision, nz, converge);
     int *wt = (int *)malloc(sizeof(int) * ((size_t)n + 1));
-    if (!wt) return 1;
+    if (!wt) { FK_ERR("%s: out of memory", who); return 1; }
     long total = 0;
     bool fit = cap > 0;
     for (int w = 0; w < n; w++) {
@@ -183,13 +183,25 @@ int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char
     const int most = total < cap ? (int)total : cap;   /* tiles of one launch */
     const size_t off_0 = al(sizeof(int) * 2 * (size_t)total), off_e = off_0 + al(sizeof(int) * (size_t)n);
     const size_t off_w = off_e + 256, bytes = off_w + fk3d_tile_edge_bytes(precision, most, nz);
-    char *m = t ? (char *)fk_dalloc(bytes, who) : NULL;
-    int e = m ? 0 : 1;
+    void *p = NULL;
+    if (t && cudaMalloc(&p, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();   /* the slabs need none of it */
+        free(t);
+        return 0;
+    }
+    char *m = (char *)p;
+    int e = t ? 0 : 1;
+    if (e) FK_ERR("%s: out of memory", who);
     if (!e) e = fk_check((int)fk_h2d(m, t, sizeof(int) * 2 * (size_t)total), who);
     if (!e) e = fk_check((int)fk_h2d(m + off_0, wt, sizeof(int) * (size_t)n), who);
     if (!e) e = fk_check((int)fk_zero(m + off_e, bytes - off_e), who);
     free(t);
-    if (e) { fk_dfree(m); return 1; }
+    if (e) {
+        fk_dfree(m);
+        free(wt);
+        pl->work_tiles = NULL;      /* the next call tries again */
+        return 1;
+    }
     pl->tile_mem = m;
     pl->dev.tiles = (const int *)m;
     pl->dev.tile0 = (const int *)(m + off_0);

@@ -25,8 +25,8 @@ int fk_slabplan_build(fk_slabplan_t *pl, int nwork, const int *nx, const int *ny
                       const int *gid, int npass, int pairing, const char *who);
 void fk_slabplan_free(fk_slabplan_t *pl);
 /* Prepare the tile schedule of a built plan (once for a precision and
- * convergence setting); have_tiles tells whether
- * every work item's tiles fit the chip at once.  Returns 0 unless memory ran
- * out. */
+ * convergence setting); have_tiles tells whether every work item's tiles fit
+ * the chip at once and the device had the memory for them (tens of MB; without,
+ * the slabs run).  Returns 0 unless a copy failed or the host's memory ran out. */
 int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who);
 #endif
