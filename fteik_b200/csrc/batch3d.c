@@ -632,6 +632,7 @@ static int tune(const char *who)
                 best_pass = m;
             }
         }
+        if (!best[6]) fk_slabplan_drop_tiles(&SB.plan);
     }
     tune_apply(best);
     SB.tune_ms[0] = best_init;

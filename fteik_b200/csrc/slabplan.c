@@ -142,15 +142,21 @@ int fk_slabplan_build(fk_slabplan_t *pl, int nwork, const int *nx, const int *ny
     return 0;
 }
 
-int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who)
+void fk_slabplan_drop_tiles(fk_slabplan_t *pl)
 {
-    const int key = 2 * precision + (converge != 0);
-    if (pl->work_tiles && pl->tile_key == key) return 0;
     fk_dfree(pl->tile_mem);
     free(pl->work_tiles);
     pl->tile_mem = NULL;
     pl->work_tiles = NULL;
     pl->have_tiles = false;
+    pl->dev.use_tiles = 0;
+}
+
+int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who)
+{
+    const int key = 2 * precision + (converge != 0);
+    if (pl->work_tiles && pl->tile_key == key) return 0;
+    fk_slabplan_drop_tiles(pl);
     pl->tile_key = key;
     const int n = pl->nwork, nz = pl->dev.max_nz;
     const int cap = fk3d_tile_capacity(precision, nz, converge);

@@ -29,4 +29,6 @@ void fk_slabplan_free(fk_slabplan_t *pl);
  * the chip at once and the device had the memory for them (tens of MB; without,
  * the slabs run).  Returns 0 unless a copy failed or the host's memory ran out. */
 int fk_slabplan_tiles(fk_slabplan_t *pl, int precision, int converge, const char *who);
+/* Give its memory back (the slabs are in use). */
+void fk_slabplan_drop_tiles(fk_slabplan_t *pl);
 #endif

@@ -28,3 +28,32 @@ def test_slabs_run_without_memory_for_the_tiles(fk, fill):  # noqa: F811
     finally:
         fk.set_slab_config(*old)
         s.free()
+
+
+def test_a_batch_on_slabs_keeps_no_tile_memory(fk):
+    """The search times the tiles; where it takes the slabs (28 sources need ten
+    launches of tiles) their scratch, 48 MB, is given back."""
+    import torch
+    grid = (60, 97, 83, 50.0, 50.0, 50.0)
+
+    def used(cfg, src):
+        old = fk.set_slab_config(*cfg)
+        try:
+            b = fk.Batch3D([grid], nsweep=2, eps=5.0, precision=4)
+            b.setVelocityModel(1, np.full((82, 96, 59), 3000.0))
+            b.setSources(1, *[np.linspace(100.0, (m - 3) * 50.0, src) for m in grid[:3]])
+            before = torch.cuda.mem_get_info()[0]
+            b.solve()
+            after = torch.cuda.mem_get_info()[0]
+            c = b.slabConfig()
+            b.finalize()
+        finally:
+            fk.set_slab_config(*old)
+        return before - after, c
+
+    for cfg in (SLABS, TILES):            # kernels loaded, the stream's pools grown
+        used(cfg, 2)
+    want, _ = used(SLABS, 28)
+    got, c = used(TILES, 28)
+    assert c["tune_runs"] > 0 and c["init_ms"] > 0.0
+    assert got - want < 16 << 20, (got, want)
