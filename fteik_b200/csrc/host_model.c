@@ -370,6 +370,8 @@ void fteik_model_setNodalVelocityModel64f(int ng, int order, const double vel[],
     fk_model.have_model = true;
 }
 
+#define SLOW_TMP_MAX ((size_t)64 << 20)   /* staging buffer kept with the grid, at most */
+
 const void *fk_model_slow_dev(int precision)
 {
     /* Upload the slowness once per model in the solve's precision. */
@@ -384,7 +386,8 @@ const void *fk_model_slow_dev(int precision)
         *slot = fk_dalloc(nelem * (size_t)precision, "fteik_model");
         if (!*slot) return NULL;
     }
-    /* the staging buffer stays with the grid: a free waits for the device */
+    /* the staging buffer stays with the grid, as a free waits for the device; a
+     * large one, whose copy takes far longer than that, is given back */
     if (!fk_model.slow_tmp) fk_model.slow_tmp = (double *)fk_dalloc(sizeof(double) * (size_t)fk_model.ncell, "fteik_model");
     double *tmp = fk_model.slow_tmp;
     if (!tmp) return NULL;
@@ -393,6 +396,10 @@ const void *fk_model_slow_dev(int precision)
                                     cudaMemcpyHostToDevice, fk_stream());
     if (!e) e = fk_pack_slowness(precision, fk_model.lis3d, nz, nx, ny, zcp, tmp, *slot, fk_stream());
     if (!e) e = (int)cudaStreamSynchronize(fk_stream());
+    if (sizeof(double) * (size_t)fk_model.ncell > SLOW_TMP_MAX) {
+        fk_dfree(tmp);
+        fk_model.slow_tmp = NULL;
+    }
     if (fk_check(e, "fteik_model: slowness upload")) return NULL;
     *ok = true;
     return *slot;
