@@ -382,17 +382,19 @@ __device__ __forceinline__ void tile_sweep(const Params &P, Smem<R> &sm, R *F, c
         R *const dst = &sm.plane[0][vy + 1][vx + 1];
         const bool writes = c <= TX + TY;
         Word<R> q[AHEAD];
-        bool dead = *((volatile int *)&sm.dead) != 0;
+        bool dead = false;
         /* a step's entry, its word loaded AHEAD steps before (in `slot`) */
         auto step = [&](int slot) {
             const bool want = (unsigned)j < Zw;
             if (!dead && !__all_sync(0xffffffffu, !want || q[slot].ok(tag))) {
                 long long it = 0;
                 do {
-                    if (++it > P.spin_limit || ((it & 63) == 0 && *((volatile int *)P.error) != 0)) {
+                    /* by vote: a lane that gave up alone would be missing in the next one */
+                    if (++it > P.spin_limit ||
+                        ((it & 63) == 0 && __any_sync(0xffffffffu, *((volatile int *)P.error) != 0))) {
                         if (c == 0) {
                             atomicCAS(P.error, 0, 4000);
-                            *((volatile int *)&sm.dead) = 1;
+                            sm.dead = 1;
                         }
                         dead = true;
                         break;
@@ -485,13 +487,13 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? 2 : 1) tile_kernel(Params
     double dmax = 0.0;
     for (int s = 0; s < 8; ++s) {
         tile_sweep<R, true, CONV>(P, sm, F, S, g, tl, mesh, s, dmax);
-        if (sm.dead) return;     /* uniform: set before the sweep's last barrier */
+        if (__syncthreads_or(sm.dead)) return;     /* all threads or none: the next sweep may set it again */
     }
     for (int pass = 0; pass < P.npass; ++pass) {
         dmax = 0.0;
         for (int s = 8 + 8 * pass; s < 16 + 8 * pass; ++s) {
             tile_sweep<R, false, CONV>(P, sm, F, S, g, tl, mesh, s, dmax);
-            if (sm.dead) return;
+            if (__syncthreads_or(sm.dead)) return;
         }
         if (CONV) {
             for (int o = 16; o > 0; o >>= 1) {
@@ -523,8 +525,7 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? 2 : 1) tile_kernel(Params
                     atomicMin(P.conv_pass + me.x, pass);
                 }
             }
-            __syncthreads();
-            if (sm.dead) return;
+            if (__syncthreads_or(sm.dead)) return;
             if (sm.stop) break;
         }
     }
