@@ -536,18 +536,25 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? 2 : 1) tile_kernel(Params
     }
 }
 
-/* Tiles of a launch: as many as fit the chip at once, 0 if none. */
+/* Tiles of a launch: as many as fit the chip at once, 0 if none.  The kernel's
+ * shared-memory limit is the device's, the same for all calls: solvers, batches
+ * and their captured graphs share the kernel. */
 template <typename R, bool CONV>
 int tile_capacity(int nz)
 {
     int dev = 0, nsm = 0, per = 0, most = 0;
     const size_t smem = tile_bytes<R>(nz);
+    cudaFuncAttributes fa;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (smem + sizeof(Smem<R>) > (size_t)most) return 0;
-    if (cudaFuncSetAttribute(tile_kernel<R, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
+    if (cudaFuncGetAttributes(&fa, tile_kernel<R, CONV>) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    const int limit = most - (int)fa.sharedSizeBytes;
+    if (limit < 0 || smem > (size_t)limit) return 0;
+    if (cudaFuncSetAttribute(tile_kernel<R, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tile_kernel<R, CONV>, NT, smem) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
