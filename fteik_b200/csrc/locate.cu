@@ -276,8 +276,11 @@ __device__ __forceinline__ void block_arrived()
  * 512 events x 64 tables x 2.46e6 points: 6.5 -> 2.1 ms a call, of which the
  * block bound takes 0.35, its preparation and the picks 0.4, the points 0.9
  * and the sample 0.2; 64 % of the issue slots are used.  CTAS to an SM: three
- * up to 48 tables (300 events x 30 x 1.1e6 points: 868 us against 940 with
- * two), above that the tables' shared memory leaves room for two. */
+ * up to 32 tables (300 events x 30 x 1.1e6 points: 868 us against 940 with
+ * two); above that the tables' shared memory (from 33 on 85 KB a CTA, its
+ * static part and the reserve included, of 228) leaves room for two, and with
+ * their registers 512 events x 33, 40, 48 tables x 266e3 points take 626, 662,
+ * 713 us instead of 648, 682, 729. */
 template <int CTAS>
 __global__ void __launch_bounds__(kBlkThreads, CTAS)
 l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, int nev, int group,
@@ -618,9 +621,12 @@ constexpr int kBoundEvents = 8, kBoundPoints = 4096;
 constexpr int kSample = 256;
 /* Blocks of points pay from about 200 events (their centres and departures
  * cost as much as some 100 events' point bounds) and on fine grids, where the
- * times change little within 32 points; above 48 tables two CTAs share an SM
- * instead of three and the grid has to be larger.  By points / by blocks, us:
- * 192 events x 269e3 points x 14, 30, 60 tables 198 / 183, 249 / 243, 387 / 412;
+ * times change little within 32 points; above 48 tables, where the blocks'
+ * centres and the warps' points are dearest, the grid has to be larger.  By
+ * points / by blocks, us: 192 events x 269e3 points x 14, 30, 60 tables
+ * 198 / 183, 249 / 243, 387 / 412; 256 events x 266e3 x 33, 40, 48 491 / 469,
+ * 504 / 502, 532 / 531 (192 events 391 / 402, 403 / 428, 432 / 455), x 410e3
+ * 600 / 441, 608 / 471, 646 / 505;
  * x 542e3 x 60 673 / 668; x 1.09e6 x 60 1311 / 1141; 60 events x 600e3 x 20
  * 183 / 207; 300 events x 99e3 x 32 210 / 250; 500 events x 256e3 x 20
  * 496 / 382. */
@@ -674,10 +680,10 @@ cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, 
     int group;
     const dim3 gb = block_grid(ngrd, nev, &group);
     const size_t smem = block_smem(ntf);
-    auto *kernel = ntf <= 48 ? l2_block_kernel<3> : l2_block_kernel<2>;
+    auto *kernel = ntf <= 32 ? l2_block_kernel<3> : l2_block_kernel<2>;
     /* the limit for the widest tables it serves: calls of other threads may set it too */
     const cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)block_smem(ntf <= 48 ? 48 : kMaxTf));
+                                                (int)block_smem(ntf <= 32 ? 32 : kMaxTf));
     if (ea != cudaSuccess) return ea;
     kernel<<<gb, kBlkThreads, smem, s>>>(
         ngrd, ldgrd, ntf, tables, nev, group, obs, wts, xn, best);
