@@ -68,6 +68,17 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long key)
 constexpr float kSlackS2 = 1.0f / 65536;   /* 2^-16 >= (3 k + 32) e */
 constexpr float kSlackObj = 1.0f / 65536;  /* 2^-16 >= (k + 36) e */
 constexpr float kSlackO2 = 1.0f / 1048576; /* 2^-20 = 16 e */
+/* The relative errors above hold while nothing underflows or overflows: squares
+ * of small terms lose at most 2^-149 each, with s3 / sum w^2 a difference of times
+ * (up to 10^4) far below kSlackMin in all, if sum w^2 itself is far above 2^-149; a
+ * sum w^2 outside [kSum2Min, kSum2Max] rules nothing out. */
+constexpr float kSlackMin = 1e-36f, kSum2Min = 1e-36f, kSum2Max = 1e36f;
+
+/* 1 / sum w^2; infinite, which makes the bound -infinity or a NaN, where it may not be used. */
+__device__ __forceinline__ float bound_scale(float sum_w2)
+{
+    return sum_w2 >= kSum2Min && sum_w2 <= kSum2Max ? 1.0f / sum_w2 : __int_as_float(0x7f800000);
+}
 
 /* Searches the points p stride, p < np = ceil(ngrd / stride).  A warp owns 64
  * points, two per lane (32 apart, so every load is 4-byte and coalesced
@@ -142,9 +153,9 @@ l2_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
             if (lane >= 2) a += up;
             up = __shfl_up_sync(0xffffffffu, a, 4);
             if (lane >= 4) a += up;
-            if (lane < kLevels) s_is2[e][lane] = a > 0.0f ? 1.0f / a : 0.0f;
+            if (lane < kLevels) s_is2[e][lane] = bound_scale(a);
             if (lane == 0) {
-                s_o2[e] = kSlackO2 * o2;
+                s_o2[e] = fmaf(kSlackO2, o2, kSlackMin);
                 s_xn[e] = xnorm[e0 + e];
                 const unsigned long long b = __ldcg(best + e0 + e);
                 s_u[e] = (unsigned)(b >> 32);            /* none yet: a NaN, which rules nothing out */
@@ -367,9 +378,9 @@ l2_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
                 for (int k = 0; k < nl; ++k) {
                     a += s_sum[k][tid].x;
                     o2 += s_sum[k][tid].y;
-                    s_is2[c0 + tid][k] = a > 0.0f ? 1.0f / a : 0.0f;
+                    s_is2[c0 + tid][k] = bound_scale(a);
                 }
-                s_o2[c0 + tid] = kSlackO2 * o2;
+                s_o2[c0 + tid] = fmaf(kSlackO2, o2, kSlackMin);
             }
             __syncthreads();
             /* the blocks: 4 of them (two packed pairs) and 2 events to a thread */
