@@ -850,6 +850,15 @@ __device__ __forceinline__ float l1_sorted_misfit(float (&r)[N], int n)
  * the same, N <= 64 (times the event's weight). */
 constexpr float kSlackL1 = 1.0f / 131072;   /* 2^-17 = 128 e */
 
+/* An event's share of what kSlackL1 applies to, so = sum |o|.  The ranked product
+ * of misfit and weight is rounded to 2^-149 at least, which moves a misfit by
+ * 2^-150 / w: less than kSlackL1 1e-15 for weights down to 1e-25; below, nothing
+ * is ruled out. */
+__device__ __forceinline__ float l1_slack_obs(float so, float w)
+{
+    return w >= 1e-25f ? so + 1e-15f : __int_as_float(0x7f800000);
+}
+
 /* Searches the points p stride; a warp owns 32 points, one a lane, and runs
  * over the events as l2_search_kernel does.  BOUND: for any t0 two picks
  * give |r_i - t0| + |r_j - t0| >= |r_i - r_j|, so the sum over disjoint pairs
@@ -914,7 +923,7 @@ l1_search_kernel(int ngrd, int ldgrd, int ntf, int stride, const float *__restri
             if (lane == 0) {
                 s_n[e] = n;
                 s_wv[e] = wv;
-                s_o[e] = so;
+                s_o[e] = l1_slack_obs(so, wv);
                 const unsigned long long b = __ldcg(best + e0 + e);
                 s_u[e] = (unsigned)(b >> 32);                /* none yet: a NaN, which rules nothing out */
                 s_best[e] = ~0ull;
@@ -1049,7 +1058,7 @@ l1_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
                 if (lane == 0) {
                     s_n[c0 + e] = cnt;
                     s_wv[c0 + e] = __uint_as_float(wv);       /* one weight per event */
-                    s_o[c0 + e] = so;
+                    s_o[c0 + e] = l1_slack_obs(so, __uint_as_float(wv));
                 }
             }
             __syncthreads();

@@ -1,6 +1,7 @@
-"""Grid search with weights whose squares leave the range of normal FP32 numbers:
-the bounds may then rule nothing out, and the optimum is still the full search's
-(the oracle's, bit for bit)."""
+"""Grid search with weights whose squares, or whose products with the misfits, leave
+the range of normal FP32 numbers: the bounds may then rule nothing out, and the
+optimum is still the full search's -- the oracle's, bit for bit (L2), or the first
+minimum of the FP32 misfits formed as in the search (L1)."""
 import numpy as np
 import pytest
 
@@ -37,3 +38,25 @@ def test_l2_weights_of_any_size(fk, scale, ntf, ngrd, nev):
     got = _locate(fk, tables, picks, wts, 2)
     for e in range(0, nev, 1 if nev < 20 else 37):
         assert tuple(v[e] for v in got) == _oracle(tables, picks[e], wts[e]), e
+
+def _l1_best(tables, picks, w):
+    r = np.sort((picks - picks.max()).astype(np.float32)[:, None] - tables, axis=0)
+    n = len(r)
+    obj = np.zeros(tables.shape[1], np.float32)
+    for i in range(n):
+        if i < n // 2:
+            obj = obj - r[i]
+        elif i >= n - n // 2:
+            obj = obj + r[i]
+    key = (obj * np.float32(w)).view(np.uint32)      # ordered as the search orders them
+    return int(np.argmin(key)) + 1
+
+
+@pytest.mark.parametrize("scale", [1e-44, 1e-42, 1e-40, 1e-38, 1e-30, 1e30, 1e37])
+@pytest.mark.parametrize("ntf,ngrd,nev", [(5, 9000, 12), (20, 9000, 12), (20, (1 << 16) + 5, 40)])
+def test_l1_weights_of_any_size(fk, scale, ntf, ngrd, nev):
+    tables = _tables(ntf, ngrd)
+    _, picks = synthetic_events(tables, nev, seed=ntf + 1)
+    got = _locate(fk, tables, picks, np.full(picks.shape, scale), 1)
+    for e in range(0, nev, 1 if nev < 20 else 7):
+        assert got[0][e] == _l1_best(tables, picks[e], scale), e
