@@ -1240,7 +1240,8 @@ __global__ void l1_at_opt_kernel(int ldgrd, int ntf, const float *__restrict__ t
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nev) return;
-    const int g = (int)(best[e] & 0xffffffffu);
+    /* weights that vanish in FP32 leave no key: every ranked misfit is zero, the first point the optimum */
+    const int g = best[e] == ~0ull ? 0 : (int)(best[e] & 0xffffffffu);
     double r[64];
     int n = 0;
     double wv = 0.0;

@@ -60,3 +60,17 @@ def test_l1_weights_of_any_size(fk, scale, ntf, ngrd, nev):
     got = _locate(fk, tables, picks, np.full(picks.shape, scale), 1)
     for e in range(0, nev, 1 if nev < 20 else 7):
         assert got[0][e] == _l1_best(tables, picks[e], scale), e
+
+
+@pytest.mark.parametrize("ngrd", [100, 5000])
+def test_l1_weights_that_vanish_in_fp32(fk, ngrd):
+    """Every ranked misfit is zero: the first point, with its FP64 values."""
+    tables = _tables(7, ngrd)
+    _, picks = synthetic_events(tables, 3, seed=5)
+    w = 1e-50
+    idx, t0, obj = _locate(fk, tables, picks, np.full(picks.shape, w), 1)
+    r = picks - tables[:, 0].astype(np.float64)
+    med = np.median(r, axis=1)
+    assert (idx == 1).all()
+    assert np.allclose(t0, med, rtol=1e-12, atol=1e-9)
+    assert np.allclose(obj / w, np.abs(r - med[:, None]).sum(1), rtol=1e-9)
