@@ -679,7 +679,7 @@ cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, 
         l2_search_kernel<NTF, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, xn, best);
         return cudaSuccess;
     }
-    const long long cs = ((ngrd + kSample - 1) / kSample + (long long)per - 1) / per;
+    const long long cs = ((ngrd + (long long)kSample - 1) / kSample + (long long)per - 1) / per;
     int schunk;
     const dim3 sgrid = point_grid(cs, nev, &schunk);
     l2_search_kernel<NTF, false><<<sgrid, kThreads, 0, s>>>(
@@ -1212,7 +1212,7 @@ cudaError_t launch_l1_search(int ngrd, int ldgrd, int ntf, const float *tables, 
         l1_search_kernel<N, false><<<grid, kThreads, 0, s>>>(ngrd, ldgrd, ntf, 1, tables, nev, chunk, obs, wts, best);
         return cudaSuccess;
     }
-    const long long cs = ((ngrd + kSample - 1) / kSample + (long long)kThreads - 1) / kThreads;
+    const long long cs = ((ngrd + (long long)kSample - 1) / kSample + (long long)kThreads - 1) / kThreads;
     int schunk;
     const dim3 sgrid = point_grid(cs, nev, &schunk);
     l1_search_kernel<N, false><<<sgrid, kThreads, 0, s>>>(
