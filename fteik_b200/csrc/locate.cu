@@ -669,7 +669,7 @@ inline dim3 block_grid(int ngrd, int nev, int *group)
 
 template <int NTF>
 cudaError_t launch_l2_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
-                      const float *xn, unsigned long long *best, cudaStream_t s)
+                             const float *xn, unsigned long long *best, cudaStream_t s)
 {
     const int per = kThreads / 32 * 64;
     const long long ctas = (ngrd + (long long)per - 1) / per;
@@ -1191,7 +1191,6 @@ l1_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
     }
 }
 
-/* One or two launches, as launch_l2_search. */
 /* Where blocks pay, as for L2; the point bound is dear here, so earlier.  By
  * points / by blocks, us: 100 events x 99e3 points x 20 tables 206 / 155, 30
  * events x 144e3 x 20 128 / 128, 10 x 99e3 x 20 81 / 99; above 32 tables (64
@@ -1200,10 +1199,10 @@ l1_block_kernel(int ngrd, int ldgrd, int ntf, const float *__restrict__ tables, 
 inline int l1_block_events(int ntf) { return ntf <= 32 ? 32 : 64; }
 inline int l1_block_points(int ntf) { return ntf <= 32 ? 1 << 16 : 1 << 18; }
 
-
+/* One or two launches, as launch_l2_search. */
 template <int N>
 cudaError_t launch_l1_search(int ngrd, int ldgrd, int ntf, const float *tables, int nev, const float *obs, const float *wts,
-                      unsigned long long *best, cudaStream_t s)
+                             unsigned long long *best, cudaStream_t s)
 {
     const long long ctas = (ngrd + (long long)kThreads - 1) / kThreads;
     int chunk;

@@ -699,7 +699,8 @@ struct PruneGeom {
     int ldgrd, ldc, ntf;
 };
 
-/* One warp per event.
+/* A CTA of one warp per event (events differ in their blocks: 0.36 ms against
+ * 0.38 with eight warps to a CTA).
  *  1. the RC best coarse runs of the tensor-core ranking on the coarse
  *     (surrogate) tables; every coarse node of them scored in FP64 on those
  *     tables; the K best coarse nodes kept;
@@ -723,34 +724,28 @@ struct PruneGeom {
  *     the exact misfit, 32 blocks at most); flag[e] = 1 when the limit stops
  *     it, and the caller searches the event exhaustively.
  * flag[e]: 0xFF for a fall-back event, else the number of blocks examined. */
-/* (a CTA per event: events differ in their blocks, 0.36 against 0.38 ms with 8) */
-constexpr int PRUNE_WARPS = 1;
-
-__global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kernel(int nev, int npart, int RC, int K, PruneGeom G,
-                             const float *__restrict__ coarse, const float *__restrict__ fine,
-                             const double *__restrict__ obs, const double *__restrict__ wts,
-                             const unsigned char *__restrict__ elig, const float *__restrict__ cand_v,
-                             const int *__restrict__ cand_i, int *__restrict__ out_idx,
-                             double *__restrict__ out_t0, double *__restrict__ out_obj,
-                             unsigned char *__restrict__ flag)
+__global__ void __launch_bounds__(32, 24)
+prune_kernel(int nev, int npart, int RC, int K, PruneGeom G, const float *__restrict__ coarse,
+             const float *__restrict__ fine, const double *__restrict__ obs, const double *__restrict__ wts,
+             const unsigned char *__restrict__ elig, const float *__restrict__ cand_v, const int *__restrict__ cand_i,
+             int *__restrict__ out_idx, double *__restrict__ out_t0, double *__restrict__ out_obj,
+             unsigned char *__restrict__ flag)
 {
-    __shared__ int s_sel[PRUNE_WARPS][32];   /* examined coarse nodes per warp */
-    __shared__ double s_o[PRUNE_WARPS][BK], s_w[PRUNE_WARPS][BK];
-    __shared__ float s_of[PRUNE_WARPS][BK];  /* shifted picks */
-    const int wib = threadIdx.x >> 5;
-    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    __shared__ int s_sel[32];    /* examined coarse nodes */
+    __shared__ double s_o[BK], s_w[BK];
+    __shared__ float s_of[BK];   /* shifted picks */
+    const int e = blockIdx.x, lane = threadIdx.x;
     if (e >= nev || !elig[e]) return;
     const long long ncoarse = (long long)G.ncz * G.ncx * G.ncy;
     const int C = npart * TOPK;
     const float *cv = cand_v + (size_t)e * C;
     const int *ci = cand_i + (size_t)e * C;
     for (int i = lane; i < BK; i += 32) {
-        s_o[wib][i] = i < G.ntf ? obs[(size_t)e * G.ntf + i] : 0.0;
-        s_w[wib][i] = i < G.ntf ? wts[(size_t)e * G.ntf + i] : 0.0;
+        s_o[i] = i < G.ntf ? obs[(size_t)e * G.ntf + i] : 0.0;
+        s_w[i] = i < G.ntf ? wts[(size_t)e * G.ntf + i] : 0.0;
     }
     __syncwarp();
-    const double *o = s_o[wib], *w = s_w[wib];
+    const double *o = s_o, *w = s_w;
     double sw = 0.0, sw2 = 0.0;
     for (int i = 0; i < G.ntf; ++i) { sw += w[i]; sw2 += w[i] * w[i]; }
     /* 1a. best coarse runs; each lane scores its point of every run */
@@ -809,7 +804,7 @@ __global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kern
         if (mi == 0x7fffffff) break;
         pvd = mv;
         pid = mi;
-        if (lane == 0) s_sel[wib][k] = mi;
+        if (lane == 0) s_sel[k] = mi;
         nsel = k + 1;
         if (k == 0) {     /* the best coarse node's origin time */
             bool own = false;
@@ -826,13 +821,13 @@ __global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kern
     float o2 = 0.0f;
     for (int i = lane; i < BK; i += 32) {
         const float v = i < G.ntf ? (float)(o[i] - tref) : 0.0f;
-        s_of[wib][i] = v;
+        s_of[i] = v;
         o2 = fmaf(v, v, o2);
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) o2 += __shfl_xor_sync(0xffffffffu, o2, s);
     __syncwarp();
-    const float *of = s_of[wib];
+    const float *of = s_of;
     const float inv_n = 1.0f / (float)G.ntf;
     const double to_var = 2.0 / (w[0] * w[0]);    /* misfit -> sum of squares */
     float ub = __int_as_float(0x7f800000);        /* above the best sum of squares so far */
@@ -849,7 +844,7 @@ __global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kern
     double best = 1.0e300, bt0 = 0.0;
     int bg = 0x7fffffff, bk = -1;
     auto scan_block = [&](int k) {
-        const int c = s_sel[wib][k];
+        const int c = s_sel[k];
         const int cz = c % G.ncz, cx = (c / G.ncz) % G.ncx, cy = c / (G.ncz * G.ncx);
         const float *const blk = fine + (size_t)c * G.ntf * nbp;
         bool scored = false;
@@ -930,7 +925,7 @@ __global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kern
             if (gz >= 0 && gx >= 0 && gy >= 0 && gz < G.nz && gx < G.nx && gy < G.ny) {
                 const int cn = gz / G.bz + G.ncz * (gx / G.bx + G.ncx * (gy / G.by));
                 bool have = false;
-                for (int k = 0; k < nsel; ++k) have |= s_sel[wib][k] == cn;
+                for (int k = 0; k < nsel; ++k) have |= s_sel[k] == cn;
                 if (!have) add = cn;
             }
         }
@@ -938,7 +933,7 @@ __global__ void __launch_bounds__(32 * PRUNE_WARPS, 24 / PRUNE_WARPS) prune_kern
         add = miss ? __shfl_sync(0xffffffffu, add, __ffs(miss) - 1) : -1;
         if (add < 0) break;
         if (nsel >= MAXB) { fb = 1; break; }
-        if (lane == 0) s_sel[wib][nsel] = add;
+        if (lane == 0) s_sel[nsel] = add;
         __syncwarp();
         scan_block(nsel);
         ++nsel;
@@ -1126,8 +1121,8 @@ extern "C" int fk_locate_prune(int nev, int npart, int rc, int k, int nz, int nx
     G.ncx = (nx + bx - 1) / bx;
     G.ncy = (ny + by - 1) / by;
     G.ldgrd = ldgrd; G.ldc = ldc; G.ntf = ntf;
-    prune_kernel<<<(nev + PRUNE_WARPS - 1) / PRUNE_WARPS, 32 * PRUNE_WARPS, 0, s>>>(nev, npart, rc, k, G, coarse, fine, obs, wts, elig,
-                                                        cand_v, cand_i, out_idx, out_t0, out_obj, flag);
+    prune_kernel<<<nev, 32, 0, s>>>(nev, npart, rc, k, G, coarse, fine, obs, wts, elig, cand_v, cand_i, out_idx, out_t0,
+                                    out_obj, flag);
     return (int)cudaGetLastError();
 }
 
