@@ -20,7 +20,9 @@
  * A point is skipped only if this bound, less the rounding errors of both
  * sides, exceeds the event's best objective so far, so the optimum, its
  * index and its ties are those of the full search.  The first best value
- * comes from a strided sample of the points.
+ * comes from a strided sample of the points.  Where FP32 ends (weights whose
+ * squares or whose products with misfits leave its normal range) the bounds
+ * allow for it or rule nothing out.
  *
  * Many events on a fine grid are bounded for 32 points at once first
  * (l2_block_kernel): over all picks the right-hand side is the square of a

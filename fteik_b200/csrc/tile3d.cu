@@ -32,9 +32,10 @@
  * of their own.  The tag's upper bits count launches, so buffers need no
  * clearing.
  *
- * Measured (one source): 128^3 in FP32, a pass's sweep 108 us against 430,
- * converged (7 passes) 8.3 ms a call against 31.5; 41 x 53 x 47 in FP64 2.4 ms
- * a call against 7.6.  A step takes 400 cycles in FP32 (bound by its 145
+ * Measured (one source): 128^3 in FP32, a pass's sweep 108 to 114 us against 430
+ * and more, converged after 3, 7 and 9 passes 4.1, 7.7 and 9.6 ms a call against
+ * 20.8, 41 and 50 (slabs, knobs 0, 1, 0, 0); 41 x 53 x 47 in FP64 2.3 ms a call
+ * against 7.6.  A step takes 400 cycles in FP32 (bound by its 145
  * instructions at one warp to a scheduler) and 1,100 in FP64 (160 FP64
  * instructions, which one warp issues every 4.4 cycles); a hand-over to the
  * next tile costs 6 to 7 steps.

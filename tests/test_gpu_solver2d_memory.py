@@ -71,3 +71,23 @@ def test_many_sources_then_a_gradient(fk, fill):
     import torch
     torch.cuda.empty_cache()
     assert np.isfinite(few).all() and few.shape[0] == ns
+
+
+@pytest.mark.parametrize("nz,nx,eps,nsweep", [(200, 300, 5.0, 2), (401, 210, 9.0, 1), (150, 512, 0.0, 3)])
+def test_both_walks_give_the_same_bits(fk, fill, nz, nx, eps, nsweep):
+    vel = _model(nz, nx, nz + nx)
+    s = fk.fteik2d()
+    s.initialize(nx, nz, 7.5, H, nsweep=nsweep, eps=eps)
+    s.setCellVelocityNatural(vel)
+    s.setSources([0.31 * (nx - 1) * 7.5], [0.63 * (nz - 1) * H])
+    s.solveSourceLSM(1)
+    want = s.getTravelTimeField()
+    s.free()
+    _first_call(fk)
+    fill(24 << 20)                        # the model planes alone take 21 MB or more
+    s.initialize(nx, nz, 7.5, H, nsweep=nsweep, eps=eps)
+    s.setCellVelocityNatural(vel)
+    s.setSources([0.31 * (nx - 1) * 7.5], [0.63 * (nz - 1) * H])
+    s.solveSourceLSM(1)
+    assert np.array_equal(s.getTravelTimeField(), want)
+    s.free()
