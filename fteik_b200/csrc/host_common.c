@@ -113,6 +113,7 @@ void *fk_dalloc(size_t bytes, const char *who)
     cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
     if (e != cudaSuccess) {
         FK_ERR("%s: cudaMalloc of %zu bytes failed (%s)", who, bytes, cudaGetErrorString(e));
+        (void)cudaGetLastError();   /* or the next launch's check would report it */
         return NULL;
     }
     return p;
